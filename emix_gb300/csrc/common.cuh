@@ -164,6 +164,7 @@ struct DerivTable {
     const DerivRowU *urows;  // n rows of the scaled form
     const double *u0s;     // ku weights of the scaled form: u0_k k_k (periodic)
     double sm1s;           // sm1 k_{n-1} (periodic)
+    const struct MmaTable *mma;   // host: the same operator for the tensor cores (null: none)
 };
 
 // Parallel cyclic reduction (PCR) followed by Thomas, for one compact

@@ -177,22 +177,9 @@ EMIX_DEV void deriv_yz_accum(const DerivTable &T, const double *__restrict__ in,
     }
 }
 
-// Body for one (virtual) block: bid = (x block, pencil row, field).
-template <int EPI>
-EMIX_DEV void deriv_yz_body(const DerivTable &T, const PencilFields &F, int nx, int nother, long s,
-                            long os, uint3 bid, int tid, int bdim) {
-    const int x = bid.x * bdim + tid;
-    const int o = bid.y;
-    if (x >= nx || o >= nother) return;
-    const long base = x + (long)o * os;
-    const int f = bid.z;
-    const double *__restrict__ in = pick(F.in, f) + base;
-    double *w = pick(F.w, f) + base;
-    double *out = pick(F.out, f) + base;
-    if constexpr (EPI == EPI_ACCUM) {
-        deriv_yz_accum(T, in, w, out, s);
-        return;
-    }
+// out = D f along one y/z pencil (element stride s), w = the forward sweep's
+// buffer
+EMIX_DEV void deriv_yz_store(const DerivTable &T, const double *__restrict__ in, double *w, double *out, long s) {
     const int n = T.n;
     const DerivRow *__restrict__ rows = T.rows;
 
@@ -283,6 +270,27 @@ EMIX_DEV void deriv_yz_body(const DerivTable &T, const PencilFields &F, int nx, 
     } else {
         for (; i >= 0; --i) row(i, false);
     }
+}
+
+// D f (EPI_STORE) or out += D f (EPI_ACCUM) along one pencil of element stride s
+template <int EPI>
+EMIX_DEV void deriv_pencil(const DerivTable &T, const double *__restrict__ in, double *w, double *out, long s) {
+    if constexpr (EPI == EPI_ACCUM)
+        deriv_yz_accum(T, in, w, out, s);
+    else
+        deriv_yz_store(T, in, w, out, s);
+}
+
+// Body for one (virtual) block: bid = (x block, pencil row, field).
+template <int EPI>
+EMIX_DEV void deriv_yz_body(const DerivTable &T, const PencilFields &F, int nx, int nother, long s,
+                            long os, uint3 bid, int tid, int bdim) {
+    const int x = bid.x * bdim + tid;
+    const int o = bid.y;
+    if (x >= nx || o >= nother) return;
+    const long base = x + (long)o * os;
+    const int f = bid.z;
+    deriv_pencil<EPI>(T, pick(F.in, f) + base, pick(F.w, f) + base, pick(F.out, f) + base, s);
 }
 
 // grid: (ceil(nx/blockDim.x), nother, nf); blockIdx.z = field

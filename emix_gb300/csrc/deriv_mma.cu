@@ -1,0 +1,769 @@
+// deriv_mma.cu -- the compact first derivative on the tensor cores
+// (tcgen05.mma, f16 operands, f32 sums in tensor memory).
+//
+// The FP64 pipe (2 lanes per clock and SM) bounds the factored Thomas sweeps
+// at 3 clocks per cell and field.  Here D f is a contraction of the dense
+// operator, which falls off so fast that 96 differences reach 16 outputs
+// (deriv_mma.cuh), and its products are formed exactly on the tensor cores:
+// each pencil's differences are turned into fixed-point numbers (relative to
+// the pencil's largest difference) of six balanced digits to the base 1024,
+// the operator into digits of the same kind, and the f32 sums of digit
+// products are integers below 2^24 and so exact (the error-free splitting of
+// K. Ozaki et al., Numerical Algorithms 59, 2012, applied to a banded
+// operator).  Products of digit orders i + j <= 5 are kept; what is dropped
+// is 2^-57 of the largest term, an FP64 sum of the same terms rounds at
+// 2^-53.
+//
+// One CTA per SM walks tiles of 128 pencils (one per tensor-memory lane), its
+// warps in four roles that meet on mbarriers:
+//   three warps read the next tile once for each pencil's largest exponent and
+//     largest difference (the first tile is shared by all);
+//   eight warps convert the tile's differences to digits, 16 rows (a group) at
+//     a time, into tensor memory, where they are the instruction's A operand;
+//   one warp issues the products of a block of 16 outputs: 28 instructions,
+//     since the operator's digits 0 .. 5-j lie next to each other and one
+//     instruction adds all products of the differences' digit j;
+//   eight warps combine the finished block's six sums per output.
+// Whole tiles while they fill every SM, the rest cut into segments of blocks.
+//
+// What bounds it: the roles are within a fifth of one another (per block of
+// 2048 outputs, of about 4300 clocks: instructions issued 2800, conversion
+// 2100 and waits, results 2700, scan 3400 per block's share); the ALU pipe is
+// 54% busy (165 instructions a cell, of which conversion 45, results 30, scan
+// 11 a row), the tensor pipe 15%: an instruction of up to 128 columns takes 80
+// clocks whatever its width, and 16 outputs a block are what tensor memory
+// holds beside the digits.  Measured, ms for 5 fields of 256^3, sweeps -> here:
+// closed x 1.001 -> 0.694, y 0.991 -> 0.577, z 0.991 -> 0.578; cyclic 1.215 ->
+// 0.704, 1.071 -> 0.709, 1.069 -> 0.712; the tank's step at 256^3 34.65 ->
+// 30.36 ms.  Error against a dense solve, 192 x 160 x 192 smooth fields, 2-norm:
+// A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 -> 9.4e-16,
+// C 5.7e-15 -> 3.4e-15.
+//
+// Pencils with infinities or NaN, or of magnitudes whose fixed-point
+// exponents would leave the FP64 range, take the scalar sweep (deriv.cuh)
+// after the tile.
+#include "deriv_mma.cuh"
+#include "tma.cuh"
+
+#include <cuda_fp16.h>
+
+namespace emix {
+namespace {
+
+__device__ int g_mma_timeouts = 0;
+
+constexpr int kMmaPencils = 128;            // per tile: the lanes of tensor memory
+constexpr int kRpt = 8;                     // rows of a group (outputs of a block) a thread takes at a time
+constexpr int kScanWarps = 3;               // warps that find the next tile's magnitudes
+constexpr int kScan = 16;                   // rows a step of theirs
+constexpr int kScanParts = 4;               // parts a pencil (y, z) is scanned in
+constexpr int kRole = 2 * kMmaPencils;      // converting threads, and as many for the results
+constexpr int kRoleWarps = kRole / 32;
+constexpr int kMmaThreads = 2 * kRole + 32 * (1 + kScanWarps);   // and the warp that drives the tensor core
+// tensor memory, in columns: two sets of f32 sums, then the digits of the last
+// groups, two f16 rows per column.  A block reads six groups and the seventh
+// is being converted; of the outer two it reads the three leading digits at
+// most, so the others are held for six groups only.
+constexpr int kAccCols = kMmaDig * kMmaRows;
+constexpr int kHighRing = 7, kLowRing = 6;
+constexpr int kHighCol = 2 * kAccCols, kLowCol = kHighCol + kHighRing * 24;
+constexpr int kTmemCols = 512;
+constexpr int kMmaWaitNs = 10000, kMmaWaitLimit = 1 << 15;   // a wait's slices, and their number
+constexpr int kXPitch = 17;                 // x pencils' staging tile: 17 rows, odd pitch
+constexpr int kXTileDoubles = kMmaPencils * kXPitch;
+static_assert(kLowCol + kLowRing * 24 <= kTmemCols, "tensor memory");
+
+// issued by the one lane with `lead` (the whole warp keeps the operands, so
+// that they stay in uniform registers)
+EMIX_DEV void mma_f16(unsigned d, unsigned a, unsigned long long b, unsigned idesc, unsigned acc, unsigned lead) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 :: "r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead) : "memory");
+}
+
+EMIX_DEV void tm_st4(unsigned addr, unsigned a, unsigned b, unsigned c, unsigned d) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+                 :: "r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+EMIX_DEV void tm_ld8(unsigned addr, float (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(addr));
+}
+
+// v 2^(62 - (E - 1023) + sh) modulo 2^64, truncated towards zero before the
+// shift by sh: below 2^61 in magnitude before it for E two above v's biased
+// exponent
+EMIX_DEV unsigned long long to_fixed(double v, int E, int sh) {
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    const int r = E - ((hi >> 20) & 0x7ff);
+    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const unsigned h = __funnelshift_l((unsigned)lo, mh, 10), l = (unsigned)lo << 10;
+    // 64-bit right shift: the funnel's shift is clamped at 32
+    const unsigned neg = (unsigned)(hi >> 31);
+    const unsigned rh = __funnelshift_rc(h, 0u, r) ^ neg;
+    const unsigned rl = __funnelshift_rc(__funnelshift_rc(l, h, r), 0u, max(r - 32, 0)) ^ neg;
+    const unsigned long long t = (((unsigned long long)rh << 32) | rl) + (neg & 1u);
+    return ((unsigned long long)__funnelshift_l((unsigned)t, (unsigned)(t >> 32), sh) << 32) | ((unsigned)t << sh);
+}
+
+// a value's high word to about 20 bits as a float (2^-126 and less as 2^-126;
+// meaningful for values whose exponents fit)
+EMIX_DEV float rough(int hi) {
+    const unsigned t = (unsigned)max(hi & 0x7fffffff, 897 << 20) * 8u - (896u << 23);
+    return __uint_as_float((t & 0x7fffffffu) | ((unsigned)hi & 0x80000000u));
+}
+
+struct Spread {          // of one pencil, or a part of it
+    int top;             // largest |high word|
+    unsigned low;        // low words, or-ed (zero test)
+    float diff;          // largest rough difference
+};
+
+// the ten-bit digits at bit P of two rows' words as two f16: the two bytes
+// they lie in, shifted down; 0x6400 | x is 1024 + x, and x carries a bias of 512
+template <int P>
+EMIX_DEV unsigned digit_pair(unsigned a, unsigned b) {
+    constexpr unsigned i = P / 8, sel = i | (i + 1) << 4 | (i + 4) << 8 | (i + 5) << 12;
+    const unsigned x = ((__byte_perm(a, b, sel) >> (P % 8)) & 0x03ff03ffu) | 0x64006400u;
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&x), __float2half2_rn(1536.0f));
+    return *reinterpret_cast<const unsigned *>(&h);
+}
+
+// digit P of a thread's rows to tensor memory
+template <int P>
+EMIX_DEV void put_digits(unsigned addr, const unsigned (&w)[kRpt]) {
+    static_assert(kRpt == 8, "one x4 store per digit");
+    tm_st4(addr, digit_pair<P>(w[0], w[1]), digit_pair<P>(w[2], w[3]), digit_pair<P>(w[4], w[5]),
+           digit_pair<P>(w[6], w[7]));
+}
+
+// one pencil's magnitudes, once known: the exponent its values are fixed to,
+// the left shift of their differences, and whether it takes the scalar sweep
+struct Scale {
+    int E, sh;
+    bool scalar;
+};
+
+EMIX_DEV Scale scale_of(const Spread &a) {
+    Scale r{1023, 0, false};
+    if (a.top == 0 && a.low == 0) return r;   // all zero
+    const int e = a.top >> 20;
+    r.scalar = e < 256 || e > 1790;
+    r.E = e + 2;
+    if (e >= 930 && e <= 1140) {
+        // differences are below B: shift them up to 63 bits
+        const float B = fmaf(a.diff, 1.01f, __uint_as_float((unsigned)(e - 896 + 1 - 18) << 23));
+        r.sh = min(max(r.E - 1023 - ((int)(__float_as_uint(B) >> 23) - 127), 0), 25);
+    }
+    return r;
+}
+
+// a tile of pencils as one thread sees it
+struct Tile {
+    const double *in;    // y, z: this thread's pencil; x: the field
+    double *out;         // likewise
+    long wofs;           // the pencil's offset in the field
+    int p0, field;
+    int b0, b1, ga, gb;  // blocks [b0, b1) of it, groups ga .. gb
+    bool live;
+};
+
+// magnitudes of the 128 x pencils from p0 of field f: P at a time, lanes along
+// the rows, kScan / P rounds of 32 rows each (P = 1: as many as it takes)
+template <int P, bool PER>
+EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, int lane, Spread *to) {
+    constexpr int C = kScan / P;
+    const int steps = P == 1 ? (n + 32 * C - 1) / (32 * C) : 1;
+    double sv[kScan], before[P];
+    int top[P];
+    unsigned low[P];
+    float diff[P], prev[P];
+    auto load = [&](int u, int st) {
+        const int r = st * 32 * C + lane;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+            const double *fp = f + (long)min(p0 + u * P + i, np - 1) * n;
+            if (st == 0) before[i] = fp[PER ? n - 1 : 0];
+#pragma unroll
+            for (int q = 0; q < C; ++q) sv[i * C + q] = fp[min(r + 32 * q, n - 1)];
+        }
+    };
+    int u = uw, st = 0;
+    if (u < kMmaPencils / P) load(u, 0);
+    while (u < kMmaPencils / P) {
+        if (st == 0) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                top[i] = 0;
+                low[i] = 0;
+                diff[i] = 0.0f;
+                prev[i] = rough(__double2hiint(before[i]));
+            }
+        }
+        int hi[kScan];
+#pragma unroll
+        for (int q = 0; q < kScan; ++q) {
+            hi[q] = __double2hiint(sv[q]);
+            low[q / C] |= (unsigned)__double2loint(sv[q]);
+        }
+        const int uu = u;
+        if (++st == steps) {
+            st = 0;
+            u += step;
+        }
+        if (u < kMmaPencils / P) load(u, st);
+#pragma unroll
+        for (int q = 0; q < kScan; ++q) {
+            const int i = q / C;
+            top[i] = max(top[i], hi[q] & 0x7fffffff);
+            const float x = rough(hi[q]);
+            const float pr = __shfl_sync(0xffffffffu, lane == 31 ? prev[i] : x, (lane + 31) & 31);
+            diff[i] = fmaxf(diff[i], fabsf(x - pr));
+            prev[i] = x;
+        }
+        if (u != uu) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const int tp = __reduce_max_sync(0xffffffffu, top[i]);
+                const unsigned lw = __reduce_or_sync(0xffffffffu, low[i]);
+                const unsigned d = __reduce_max_sync(0xffffffffu, __float_as_uint(diff[i]));   // not negative
+                if (lane == 0) to[uu * P + i] = Spread{tp, lw, __uint_as_float(d)};
+            }
+        }
+    }
+}
+
+// XAX: pencils along x (rows contiguous, brought through a shared tile);
+// otherwise along y or z (pencils contiguous along x)
+template <bool XAX, int EPI, bool PER>
+__global__ void __launch_bounds__(kMmaThreads, 1)
+k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTable M,
+            const __grid_constant__ PencilFields F, int np, int ntile, int nf, int whole, int segs, int nx,
+            long s, long os) {
+    extern __shared__ __align__(1024) unsigned char dyn[];
+    __shared__ unsigned s_tmem;
+    __shared__ int s_fail;
+    // full[a]: the tensor core has finished a block in sum buffer a; drained[a]:
+    // all warps have read it; conv[q]: group q (mod 8) is in tensor memory;
+    // done[b]: block b (mod 8) is finished, for the converting warps, which lag
+    // by up to five blocks at a tile's end; scaled[t]: tile t's (mod 2)
+    // magnitudes are in s_part; read[t]: every warp that wants them has them
+    __shared__ __align__(8) unsigned long long s_full[2], s_drained[2], s_conv[8], s_done[8],
+        s_scaled[2], s_read[2];
+    __shared__ Spread s_part[2][kScanParts][kMmaPencils];   // by the tile's parity
+    __shared__ unsigned char s_scalar[kMmaPencils];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = T.n;
+
+    if (tid == 0) {
+        s_fail = 0;
+        for (int q = 0; q < 2; ++q) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_full[q])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_drained[q])), "r"(kRoleWarps) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_scaled[q])), "r"(kScanWarps) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_read[q])), "r"(2 * kRoleWarps) : "memory");
+        }
+        for (int q = 0; q < 8; ++q) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_conv[q])), "r"(kRoleWarps) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_done[q])) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(smem_u32(&s_tmem)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(M.b);
+        uint4 *dst = reinterpret_cast<uint4 *>(dyn);
+        for (int q = tid; q < M.ntype * (kMmaTypeBytes / 16); q += kMmaThreads) dst[q] = src[q];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // all columns were asked for, so they begin at 0: a constant, which keeps
+    // the tensor-core instructions' operands in uniform registers
+    constexpr unsigned tm = 0;
+    if (s_tmem != tm && tid == 0) s_fail = 1;
+    const int nblk = M.nblk;
+    const int g0 = PER ? -2 : 0;                                   // first and last group of a tile
+    const int g1 = PER ? nblk + 2 : (n + 6) / kMmaRows;
+    const int jobs = whole + (ntile * nf - whole) * segs;
+    bool ok = true;                                                // false: a wait ran out; nothing is stored any more
+
+    // bounded wait; once one has run out no further one is waited for, and
+    // the loops below run out by themselves
+    auto wait = [&](unsigned long long *bar, unsigned parity) {
+        if (!ok) return;   // the same in all lanes
+        const unsigned addr = smem_u32(bar);
+        for (int it = 0; it < kMmaWaitLimit; ++it) {
+            unsigned done;
+            asm volatile("{\n\t.reg .pred p;\n\t"
+                         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+                         "selp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(done) : "r"(addr), "r"(parity), "r"(kMmaWaitNs) : "memory");
+            if (__all_sync(0xffffffffu, done)) return;
+            if (__any_sync(0xffffffffu, *(volatile int *)&s_fail)) break;
+        }
+        *(volatile int *)&s_fail = 1;
+        ok = false;
+    };
+    auto arrive = [&](unsigned long long *bar) {
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
+    };
+    auto row_sync = [](int id) { asm volatile("bar.sync %0, %1;" :: "r"(id), "n"(kRole) : "memory"); };
+
+    // row of a pencil: wrapped (cyclic), or clamped to the ends, where the
+    // repeated value makes the differences beyond them zero
+    auto row_of = [&](int k) {
+        if constexpr (PER) {
+            while (k < 0) k += n;
+            while (k >= n) k -= n;
+            return k;
+        }
+        return min(max(k, 0), n - 1);
+    };
+    // job: a whole tile, or (from `whole` on) one of `segs` segments of one
+    auto tile_of = [&](int job, int slot_p) {
+        Tile t;
+        int id = job, seg = 0, cut = 1;
+        if (job >= whole) {
+            id = whole + (job - whole) / segs;
+            seg = (job - whole) % segs;
+            cut = segs;
+        }
+        t.b0 = nblk * seg / cut;
+        t.b1 = nblk * (seg + 1) / cut;
+        t.ga = max(g0, t.b0 - 2);
+        t.gb = min(g1, t.b1 + 2);
+        t.field = id / ntile;
+        t.p0 = (id - t.field * ntile) * kMmaPencils;
+        const int p = min(t.p0 + slot_p, np - 1);
+        t.live = t.p0 + slot_p < np;
+        t.wofs = XAX ? (long)p * n : (long)(p % nx) + (long)(p / nx) * os;
+        t.in = pick(F.in, t.field) + (XAX ? 0 : t.wofs);
+        t.out = pick(F.out, t.field) + (XAX ? 0 : t.wofs);
+        return t;
+    };
+
+    // magnitudes of a tile's pencils into s_part[buf]: this warp takes units
+    // uw, uw + step, ...; kScan values a lane and step, loaded a step ahead
+    auto scan_tile = [&](int job, int buf, int uw, int step) {
+        if constexpr (!XAX) {
+            // units of 32 pencils (lanes) by a part of the rows
+            const int part = (n + kScanParts - 1) / kScanParts, steps = (part + kScan - 1) / kScan;
+            double sv[kScan], before = 0.0;    // before: the value before the unit's first row
+            const double *fp = nullptr;
+            int ra = 0, rb = 0, top = 0;
+            unsigned low = 0;
+            float diff = 0.0f, prev = 0.0f;
+            auto load = [&](int u, int st) {
+                if (st == 0) {
+                    fp = tile_of(job, (u & 3) * 32 + lane).in;
+                    ra = min((u >> 2) * part, n - 1);
+                    rb = min(ra + part, n) - 1;
+                    before = fp[(long)row_of(ra - 1) * s];
+                }
+                const int r = ra + st * kScan;
+                const double *q0 = fp + (long)r * s;
+                if (r + kScan <= n) {
+#pragma unroll
+                    for (int q = 0; q < kScan; ++q) sv[q] = q0[q * s];
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kScan; ++q) sv[q] = fp[(long)min(r + q, rb) * s];
+                }
+            };
+            int u = uw, st = 0;
+            if (u < 4 * kScanParts) load(u, 0);
+            while (u < 4 * kScanParts) {
+                if (st == 0) {
+                    top = 0;
+                    low = 0;
+                    diff = 0.0f;
+                    prev = rough(__double2hiint(before));
+                }
+                int hi[kScan];
+#pragma unroll
+                for (int q = 0; q < kScan; ++q) {
+                    hi[q] = __double2hiint(sv[q]);
+                    low |= (unsigned)__double2loint(sv[q]);
+                }
+                const int uu = u;
+                if (++st == steps) {
+                    st = 0;
+                    u += step;
+                }
+                if (u < 4 * kScanParts) load(u, st);
+#pragma unroll
+                for (int q = 0; q < kScan; ++q) {
+                    top = max(top, hi[q] & 0x7fffffff);
+                    const float x = rough(hi[q]);
+                    diff = fmaxf(diff, fabsf(x - prev));
+                    prev = x;
+                }
+                if (u != uu) s_part[buf][uu >> 2][(uu & 3) * 32 + lane] = Spread{top, low, diff};
+            }
+        } else {
+            const Tile tl = tile_of(job, 0);
+            Spread *to = s_part[buf][0];
+            if (n <= 32 * (kScan / 8)) scan_x<8, PER>(tl.in, tl.p0, np, n, uw, step, lane, to);
+            else if (n <= 32 * (kScan / 4)) scan_x<4, PER>(tl.in, tl.p0, np, n, uw, step, lane, to);
+            else if (n <= 32 * (kScan / 2)) scan_x<2, PER>(tl.in, tl.p0, np, n, uw, step, lane, to);
+            else scan_x<1, PER>(tl.in, tl.p0, np, n, uw, step, lane, to);
+        }
+    };
+    constexpr int kPencilWarps = 2 * kRoleWarps + kScanWarps;   // all but the tensor core's
+    if (warp != 2 * kRoleWarps) {
+        // the first tile's, by all of them
+        scan_tile(blockIdx.x, 0, warp < 2 * kRoleWarps ? warp : warp - 1, kPencilWarps);
+        asm volatile("bar.sync 3, %0;" :: "n"(32 * kPencilWarps) : "memory");
+    }
+
+    if (warp == 2 * kRoleWarps) {
+        // ---- the tensor core's warp ----------------------------------------
+        {
+            const unsigned leader = lane == 0;
+            int B = 0, first = 0;     // block, and the tile's first group, counted over the tiles
+            int seen = 0;             // groups known to be in tensor memory
+            for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
+                const Tile jt = tile_of(job, 0);
+                for (int b = jt.b0; b < jt.b1; ++b, ++B) {
+                    for (const int need = first + min(b + 3, jt.gb) - jt.ga; seen <= need; ++seen)
+                        wait(&s_conv[seen & 7], (unsigned)(seen >> 3) & 1);
+                    if (B >= 2) wait(&s_drained[B & 1], (unsigned)((B - 2) >> 1) & 1);
+                    if (!ok) continue;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const int ty = b < M.nlow ? b : (b >= nblk - M.nhigh ? M.ntype - (nblk - b) : M.nlow);
+                    const unsigned base = smem_u32(dyn) + (unsigned)(ty * kMmaTypeBytes);
+                    // the K-major operand without swizzle: 8 x 16-byte core
+                    // matrices, 128 bytes apart along the rows, kMmaStack x 16
+                    // along the columns
+                    constexpr unsigned long long desc0 =
+                        (1ull << 46) | ((unsigned long long)(128 >> 4) << 32) |
+                        ((unsigned long long)((kMmaStack * 16) >> 4) << 16);
+                    const unsigned sums = tm + (unsigned)(B & 1) * kAccCols;
+#pragma unroll
+                    for (int q = 0; q < kMmaWin; ++q) {
+                        const int w = q == 0 ? 2 : (q <= 2 ? q - 1 : q);   // the block's own group first
+                        constexpr int kLead[kMmaWin] = {kMmaLead0, kMmaLead1, 0, 0, kMmaLead1, kMmaLead0};
+                        const int lead = kLead[w], g = b - 2 + w;
+                        if (g < jt.ga || g > jt.gb) continue;
+                        const unsigned c = (unsigned)(first + g - jt.ga);
+                        const unsigned ah = tm + kHighCol + (c % kHighRing) * 24, al = tm + kLowCol + (c % kLowRing) * 24;
+                        const unsigned bb = base + w * kMmaGroupBytes + lead * (kMmaRows * 16);
+                        const unsigned long long desc = desc0 | ((bb >> 4) & 0x3fff);
+#pragma unroll
+                        for (int j = 0; j < kMmaDig - lead; ++j) {
+                            const unsigned idesc = (1u << 4) | ((unsigned)((kMmaDig - lead - j) * kMmaRows >> 3) << 17) |
+                                                   ((kMmaPencils >> 4) << 24);
+                            mma_f16(sums + (lead + j) * kMmaRows, j < 3 ? ah + j * 8 : al + (j - 3) * 8, desc, idesc,
+                                    !(q == 0 && j == 0), leader);
+                        }
+                    }
+                    __syncwarp();
+                    if (leader)
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+                                     "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];"
+                                     :: "r"(smem_u32(&s_full[B & 1])), "r"(smem_u32(&s_done[B & 7])) : "memory");
+                }
+                first += jt.gb - jt.ga + 1;
+            }
+        }
+    } else if (warp > 2 * kRoleWarps) {
+        // ---- magnitudes of the tiles' pencils, one tile ahead ------------------
+        int t = 1;
+        for (int job = blockIdx.x + gridDim.x; job < jobs; job += gridDim.x, ++t) {
+            if (t >= 2) wait(&s_read[t & 1], (unsigned)((t - 2) >> 1) & 1);   // s_part's turn
+            scan_tile(job, t & 1, warp - 2 * kRoleWarps - 1, kScanWarps);
+            arrive(&s_scaled[t & 1]);
+        }
+    } else {
+        // ---- the pencils' warps: converting, or the results --------------------
+        const bool results = warp >= kRoleWarps;
+        const int rtid = results ? tid - kRole : tid, rwarp = results ? warp - kRoleWarps : warp;
+        const int quarter = warp & 3;                     // tensor-memory lanes 32 quarter ..
+        const int rg = rwarp >> 2;                        // rows kRpt rg .. of a group or block
+        const int slot_p = quarter * 32 + lane;           // this thread's pencil in the tile
+        const unsigned tml = tm + ((unsigned)(quarter * 32) << 16);
+        double *xin = reinterpret_cast<double *>(dyn + (size_t)M.ntype * kMmaTypeBytes);
+        double *xout = xin + 2 * kXTileDoubles;
+        // this thread's pencil of tile t, once its magnitudes are known
+        auto scale_wait = [&](int t) {
+            if (t > 0) wait(&s_scaled[t & 1], (unsigned)((t - 1) >> 1) & 1);
+            Spread a = s_part[t & 1][0][slot_p];
+            if constexpr (!XAX) {
+#pragma unroll
+                for (int q = 1; q < kScanParts; ++q) {
+                    const Spread b = s_part[t & 1][q][slot_p];
+                    a.top = max(a.top, b.top);
+                    a.low |= b.low;
+                    a.diff = fmaxf(a.diff, b.diff);
+                }
+            }
+            arrive(&s_read[t & 1]);
+            return scale_of(a);
+        };
+        if (!results) {
+            // ---- a group's rows to digits, loaded one group ahead ---------------
+            double v[kRpt + 1];   // y, z: the thread's rows; x: staged values
+            auto load = [&](const Tile &t, int g) {
+                const int k = kMmaRows * g - 8;
+                if constexpr (!XAX) {
+                    if (k >= 0 && k + kMmaRows < n) {
+                        const double *fp = t.in + (long)(k + kRpt * rg) * s;
+#pragma unroll
+                        for (int q = 0; q <= kRpt; ++q) v[q] = fp[q * s];
+                    } else {
+#pragma unroll
+                        for (int q = 0; q <= kRpt; ++q) v[q] = t.in[(long)row_of(k + kRpt * rg + q) * s];
+                    }
+                } else {
+                    const int row = row_of(k + (rtid & 15));
+#pragma unroll
+                    for (int q = 0; q < kRpt; ++q)
+                        v[q] = t.in[(long)min(t.p0 + (rtid >> 4) + (kRole / 16) * q, np - 1) * n + row];
+                    if (rtid < kMmaPencils) v[kRpt] = t.in[(long)min(t.p0 + rtid, np - 1) * n + row_of(k + 16)];
+                }
+            };
+            auto stage = [&](int c) {   // x: into the tile of group c
+                double *t = xin + (c & 1) * kXTileDoubles;
+#pragma unroll
+                for (int q = 0; q < kRpt; ++q) t[((rtid >> 4) + (kRole / 16) * q) * kXPitch + (rtid & 15)] = v[q];
+                if (rtid < kMmaPencils) t[rtid * kXPitch + 16] = v[kRpt];
+            };
+            auto convert = [&](int c, const Scale &sc) {
+                unsigned w1[kRpt], w2[kRpt];
+                const double *t = xin + (c & 1) * kXTileDoubles + slot_p * kXPitch + kRpt * rg;
+                unsigned long long a = to_fixed(XAX ? t[0] : v[0], sc.E, sc.sh);
+#pragma unroll
+                for (int q = 0; q < kRpt; ++q) {
+                    const unsigned long long b = to_fixed(XAX ? t[q + 1] : v[q + 1], sc.E, sc.sh);
+                    // digits at bits 4 + 10 j, biased by 512; half of the bits dropped below
+                    const unsigned long long y = b - a + 0x8020080200802008ull;
+                    a = b;
+                    w1[q] = (unsigned)(y >> 32);
+                    w2[q] = (unsigned)(y >> 4);
+                }
+                const unsigned ah = tml + kHighCol + (unsigned)(c % kHighRing) * 24 + rg * (kRpt / 2);
+                const unsigned al = tml + kLowCol + (unsigned)(c % kLowRing) * 24 + rg * (kRpt / 2);
+                put_digits<22>(ah, w1);
+                put_digits<12>(ah + 8, w1);
+                put_digits<2>(ah + 16, w1);
+                put_digits<20>(al, w2);
+                put_digits<10>(al + 8, w2);
+                put_digits<0>(al + 16, w2);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                arrive(&s_conv[c & 7]);
+            };
+
+            int c = 0, done = 0, t = 0, B = 0;   // groups, finished blocks, jobs, the job's first block
+            int job = blockIdx.x;
+            Tile cur = tile_of(job, slot_p), last = cur;
+            // the last block (counted over the jobs) that reads group `pos` of a
+            // job, `reach` groups behind it at most; of one before the previous
+            // job, the last of that
+            auto last_use = [&](int pos, int reach) {
+                if (pos >= 0) return B + min(cur.ga + pos + reach, cur.b1 - 1) - cur.b0;
+                const int Bl = B - (last.b1 - last.b0);
+                if (t == 0) return -1;
+                pos += last.gb - last.ga + 1;
+                return pos >= 0 ? Bl + min(last.ga + pos + reach, last.b1 - 1) - last.b0 : Bl - 1;
+            };
+            load(cur, cur.ga);
+            for (; job < jobs; job += gridDim.x, ++t) {
+                const Scale sc = scale_wait(t);
+                const bool more = job + (int)gridDim.x < jobs;
+                Tile nxt = cur;
+                if (more) nxt = tile_of(job + gridDim.x, slot_p);
+                const int ng = cur.gb - cur.ga + 1;
+                for (int k = 0; k < ng; ++k, ++c) {
+                    // the rings' places are free once the blocks that read them are done
+                    const int need = max(last_use(k - kHighRing, 2), last_use(k - kLowRing, 1));
+                    if constexpr (XAX) {
+                        stage(c);
+                        row_sync(1);
+                        if (k + 1 < ng) load(cur, cur.ga + k + 1);
+                        else if (more) load(nxt, nxt.ga);
+                    }
+                    for (; done <= need; ++done) wait(&s_done[done & 7], (unsigned)(done >> 3) & 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    convert(c, sc);
+                    if constexpr (!XAX) {
+                        if (k + 1 < ng) load(cur, cur.ga + k + 1);
+                        else if (more) load(nxt, nxt.ga);
+                    }
+                }
+                B += cur.b1 - cur.b0;
+                last = cur;
+                cur = nxt;
+            }
+        } else {
+            // sums of the digit orders 0..5 combined exactly (weights 2^42, 2^32,
+            // 2^22, 2^12, 2^2 and 2^-8), then scaled
+            auto combine = [](const float (&acc)[kMmaDig][kRpt], int q, int escale) {
+                const int a0 = __float2int_rn(acc[0][q]), a1 = __float2int_rn(acc[1][q]);
+                const int a2 = __float2int_rn(acc[2][q]), a3 = __float2int_rn(acc[3][q]);
+                const int a4 = __float2int_rn(acc[4][q]), a5 = __float2int_rn(acc[5][q]);
+                long long r = (long long)(a4 * 4 + (a5 >> 8));
+                r += (long long)a3 * 4096;
+                r += (long long)a2 * (1 << 22);
+                const unsigned hi = (unsigned)(r >> 32) + (unsigned)(a0 * 1024 + a1);
+                const double d = (double)(long long)(((unsigned long long)hi << 32) | (unsigned)r);
+                const int dh = __double2hiint(d);
+                return __hiloint2double(dh ? dh + escale : 0, __double2loint(d));
+            };
+
+            // ---- the stream of blocks ----------------------------------------------
+            int B = 0, t = 0;
+            for (int job = blockIdx.x; job < jobs; job += gridDim.x, ++t) {
+                const Tile cur = tile_of(job, slot_p);
+                const Scale sc = scale_wait(t);
+                const int escale = (sc.E - 1023 - M.se - sc.sh) * (1 << 20);
+                if (XAX && rg == 0) s_scalar[slot_p] = sc.scalar;
+                for (int b = cur.b0; b < cur.b1; ++b, ++B) {
+                    const int row = kMmaRows * b + kRpt * rg;
+                    double old[kRpt];
+                    if constexpr (EPI == EPI_ACCUM && !XAX) {
+#pragma unroll
+                        for (int q = 0; q < kRpt; ++q) old[q] = cur.out[(long)min(row + q, n - 1) * s];
+                    }
+                    wait(&s_full[B & 1], (unsigned)(B >> 1) & 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    float acc[kMmaDig][kRpt];
+#pragma unroll
+                    for (int j = 0; j < kMmaDig; ++j)
+                        tm_ld8(tml + (unsigned)(B & 1) * kAccCols + j * kMmaRows + kRpt * rg, acc[j]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    // the sums are not touched before the wait
+#pragma unroll
+                    for (int j = 0; j < kMmaDig; ++j)
+                        asm volatile("" : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3]),
+                                          "+f"(acc[j][4]), "+f"(acc[j][5]), "+f"(acc[j][6]), "+f"(acc[j][7]));
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    arrive(&s_drained[B & 1]);
+                    if constexpr (!XAX) {
+                        if (cur.live && !sc.scalar && ok) {
+                            double *o = cur.out + (long)row * s;
+                            if (row + kRpt <= n) {
+#pragma unroll
+                                for (int q = 0; q < kRpt; ++q) {
+                                    double r = combine(acc, q, escale);
+                                    if constexpr (EPI == EPI_ACCUM) r += old[q];
+                                    o[q * s] = r;
+                                }
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < kRpt; ++q) {
+                                    double r = combine(acc, q, escale);
+                                    if constexpr (EPI == EPI_ACCUM) r += old[q];
+                                    if (row + q < n) o[q * s] = r;
+                                }
+                            }
+                        }
+                    } else {
+                        double *tl = xout + (B & 1) * kXTileDoubles;
+#pragma unroll
+                        for (int q = 0; q < kRpt; ++q) tl[slot_p * kXPitch + kRpt * rg + q] = combine(acc, q, escale);
+                        row_sync(2);
+                        // the block's tile to memory, rows along the lanes
+                        const int frow = kMmaRows * b + (rtid & 15);
+                        double *o = cur.out + (long)(cur.p0 + (rtid >> 4)) * n + frow;
+#pragma unroll
+                        for (int q = 0; q < kRpt; ++q) {
+                            const int pp = (rtid >> 4) + (kRole / 16) * q;
+                            if (frow < n && cur.p0 + pp < np && !s_scalar[pp] && ok) {
+                                double r = tl[pp * kXPitch + (rtid & 15)];
+                                if (EPI == EPI_ACCUM) r += *o;
+                                *o = r;
+                            }
+                            o += (long)(kRole / 16) * n;
+                        }
+                    }
+                }
+                // the pencils outside the fixed-point range
+                if (rg == 0 && sc.scalar && cur.live && ok && cur.b0 == 0) {
+                    const long x = XAX ? cur.wofs : 0;
+                    deriv_pencil<EPI>(T, cur.in + x, pick(F.w, cur.field) + cur.wofs, cur.out + x, s);
+                }
+                if constexpr (XAX) row_sync(2);   // s_scalar is free
+            }
+        }
+    }
+    // a wait that ran out: counted; tensor memory goes only after what the
+    // tensor core still has in flight (bounded)
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (s_fail) {
+        if (tid == 0) atomicAdd(&g_mma_timeouts, 1);
+        for (int q = 0; q < 1 << 16; ++q) __nanosleep(256);
+    }
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(kTmemCols));
+}
+
+template <bool XAX, int EPI, bool PER>
+int launch(const DerivTable &T, const MmaTable &M, const PencilFields &F, int nf, int np, int nx, long s, long os,
+           cudaStream_t st) {
+    // tensor memory is taken whole: at least 116 KB of shared memory keeps a
+    // second CTA off the SM
+    size_t shm = (size_t)M.ntype * kMmaTypeBytes + (XAX ? 4 * kXTileDoubles * sizeof(double) : 0);
+    if (shm < 120 * 1024) shm = 120 * 1024;
+    auto kernel = k_deriv_mma<XAX, EPI, PER>;
+    EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+    const int ntile = (np + kMmaPencils - 1) / kMmaPencils, tiles = ntile * nf, sms = device_sms();
+    // whole tiles while they fill every SM; what is left is cut into the
+    // number of segments (each with five more groups to convert) that ends
+    // first
+    const int whole = tiles / sms * sms, rest = tiles - whole;
+    int segs = 1;
+    long best = -1;
+    for (int c = 1; rest > 0 && c <= M.nblk && c <= 64; ++c) {
+        const long rounds = ((long)rest * c + sms - 1) / sms, t = rounds * ((M.nblk + c - 1) / c + 6);
+        if (best < 0 || t < best) { best = t; segs = c; }
+    }
+    const long jobs = whole + (long)rest * segs;
+    const int grid = (int)(jobs < sms ? jobs : sms);
+    kernel<<<grid, kMmaThreads, shm, st>>>(T, M, F, np, ntile, nf, whole, segs, nx, s, os);
+    EMIX_CUDA_TRY(cudaGetLastError());
+    return EMIX_OK;
+}
+
+template <bool XAX>
+int launch(int epi, const DerivTable &T, const MmaTable &M, const PencilFields &F, int nf, int np, int nx, long s,
+           long os, cudaStream_t st) {
+    if (M.periodic)
+        return epi == EPI_STORE ? launch<XAX, EPI_STORE, true>(T, M, F, nf, np, nx, s, os, st)
+                                : launch<XAX, EPI_ACCUM, true>(T, M, F, nf, np, nx, s, os, st);
+    return epi == EPI_STORE ? launch<XAX, EPI_STORE, false>(T, M, F, nf, np, nx, s, os, st)
+                            : launch<XAX, EPI_ACCUM, false>(T, M, F, nf, np, nx, s, os, st);
+}
+
+} // namespace
+
+int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
+                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st) {
+    PencilFields F{};
+    for (int f = 0; f < nf; ++f) {
+        F.in[f] = in[f];
+        F.w[f] = w[f];
+        F.out[f] = out[f];
+    }
+    const int nother = axis == 0 ? 0 : (axis == 1 ? nz : ny);
+    if (axis == 0) return launch<true>(epi, T, M, F, nf, ny * nz, nx, 1, 0, st);
+    const long s = axis == 1 ? (long)nx : (long)nx * ny, os = axis == 1 ? (long)nx * ny : (long)nx;
+    return launch<false>(epi, T, M, F, nf, nx * nother, nx, s, os, st);
+}
+
+int deriv_mma_timeouts(int *count) {
+    EMIX_CUDA_TRY(cudaMemcpyFromSymbol(count, g_mma_timeouts, sizeof(int)));
+    return EMIX_OK;
+}
+
+} // namespace emix

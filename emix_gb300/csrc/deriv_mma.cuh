@@ -1,0 +1,72 @@
+// deriv_mma.cuh -- the compact first derivative on the tensor cores
+// (deriv_mma.cu): exact fixed-point digits of the pencils times exact digits
+// of the dense operator.
+#pragma once
+
+#include "deriv.cuh"
+
+namespace emix {
+
+// The operator D = A^{-1} B / h acting on first differences: with
+// d_k = f_{k+1} - f_k, (D f)_i = sum_k E_{ik} d_k, E_{ik} = sum_{m>k} D_{im}
+// (the rows of D sum to zero).  |E_{ik}| falls by the root of the scheme's
+// characteristic polynomial (0.38 or 0.27) per row away from the diagonal:
+// 2^-55 of its largest entry 40 rows away, where it is cut (what is cut off is
+// added to the last entry kept, so that row sums, and with them the
+// derivative of a linear function, stay exact).
+//
+// Outputs go in blocks of 16 rows.  Block b reads the differences
+// 16b-40 .. 16b+55, in six groups of 16: group g holds 16g-8 .. 16g+7, block b
+// reads groups b-2 .. b+3.  Away from the ends every block has the same
+// entries, so a table holds few distinct block types (at most 8; one for the
+// cyclic scheme).
+//
+// Entries are fixed-point numbers of kMmaDig balanced digits to the base 1024
+// (60 bits): E 2^sE = sum_i D_i 1024^(kMmaDig-1-i), -512 <= D_i <= 511, held
+// as f16.  `b` has, per type, group and 8 columns of the group, the digits of
+// 16 rows, i-major (kMmaDig x 16 rows of 8 f16: the no-swizzle K-major
+// operand of tcgen05.mma).
+constexpr int kMmaDig = 6;
+constexpr int kMmaRows = 16;                                    // outputs of a block, differences of a group
+constexpr int kMmaWin = 6;                                      // groups a block reads
+constexpr int kMmaStack = kMmaDig * kMmaRows;                   // operand rows of a group
+constexpr int kMmaGroupBytes = 2 * kMmaStack * 16;              // one group of one type
+constexpr int kMmaTypeBytes = kMmaWin * kMmaGroupBytes;
+constexpr int kMmaMaxTypes = 8;
+// leading digits of the entries that vanish over a block's outer two groups
+// (24 rows away and more: below 2^-30) and over the two within
+constexpr int kMmaLead0 = 3, kMmaLead1 = 1;
+constexpr int kMmaMaxBlocks = kTableMaxN / kMmaRows;
+
+struct MmaTable {
+    int n, periodic;
+    int nblk;             // blocks of 16 outputs
+    int ntype;
+    int nlow, nhigh;      // blocks of their own type at the ends; type nlow is the interior's
+    int se;               // scale exponent of the entries
+    const unsigned short *b;   // ntype x kMmaTypeBytes, f16
+};
+
+// Tensor-core table of (scheme, n, sign h) (kept for the life of the
+// process); null below kMmaMinN rows and where the operator does not fit the
+// form above (the callers then keep the sweeps).
+int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out);
+
+// Whether a derivative goes to the tensor cores: by the length of its
+// pencils.  Measured against the sweeps (us a launch, 3 or 5 fields, closed /
+// cyclic): n = 32: x 17 / 21 -> 16 / 18 at 32^3 but 134 -> 200 at 32 x 128 x
+// 512, y and z 16 / 19 -> 16 / 19; n = 40: 26 / 33 -> 21 / 21, 22 / 25 -> 20 / 23;
+// n = 64: 36 / 47 -> 29 / 34, 33 / 38 -> 26 / 36; n = 256: 1001 / 1215 -> 694 /
+// 704, 991 / 1070 -> 577 / 710.  Shorter pencils have more blocks at an end and
+// groups to convert per output than the sweeps have to lose.
+constexpr int kMmaMinN = 40;
+inline bool deriv_on_mma(const DerivTable &T) { return T.mma != nullptr; }
+
+// launch_deriv on the tensor cores
+int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
+                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st);
+
+// blocks that gave up a bounded wait since the library was loaded
+int deriv_mma_timeouts(int *count);
+
+} // namespace emix

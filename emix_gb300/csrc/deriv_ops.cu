@@ -6,7 +6,7 @@
 // solver/cuDivergence.cu:124-187).  Here the device-pointer forms allocate
 // nothing but cached scratch, and the host-pointer forms keep a grow-only
 // device workspace per device so repeated calls pay only the copies.
-#include "deriv.cuh"
+#include "deriv_mma.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -55,6 +55,8 @@ int launch_deriv(const DerivTable &T, int axis, int epi, int nf, const double *c
     if (nf < 1 || nf > kMaxFields) return EMIX_ERR_ARG;
     const int n = axis == 0 ? nx : (axis == 1 ? ny : nz);
     if (T.n != n) return EMIX_ERR_ARG;
+    if (deriv_on_mma(T))
+        return launch_deriv_mma(T, *T.mma, axis, epi, nf, in, w, out, nx, ny, nz, st);
     PencilFields F{};
     for (int f = 0; f < nf; ++f) {
         F.in[f] = in[f];

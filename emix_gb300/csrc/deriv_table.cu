@@ -14,7 +14,10 @@
 //   BPER src/MSVSingle/derivada_incomp.f90:192-206 (rows), :231-247 (RHS, cyclic)
 //   C    src/Schemes/derivCompact.cu:90-99 (RHS), :162-190 (rows)
 #include "common.cuh"
+#include "deriv_mma.cuh"
 
+#include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -209,6 +212,7 @@ std::map<TableKey, DerivTable> g_tables;   // device buffers live until process 
 } // namespace
 
 int get_table_signed(int scheme, int n, double h, double sign, DerivTable *out);
+int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out);
 
 int get_deriv_table(int scheme, int n, double h, DerivTable *out) {
     if (!(h > 0.0)) return EMIX_ERR_ARG;
@@ -274,6 +278,8 @@ int get_table_signed(int scheme, int n, double h, double sign, DerivTable *out) 
     t.zz = t.u0 + n;
     t.urows = reinterpret_cast<const DerivRowU *>(t.zz + n);
     t.u0s = t.zz + 5 * (size_t)n;
+    rc = get_mma_table(scheme, n, h, sign, &t.mma);
+    if (rc) return rc;
     g_tables[key] = t;
     *out = t;
     return EMIX_OK;
@@ -544,6 +550,252 @@ int get_deriv_t_table(int scheme, int n, double h, DerivTTable *out) {
     std::lock_guard<std::mutex> lock(g_t_mu);
     g_t_tables[key] = t;
     *out = t;
+    return EMIX_OK;
+}
+
+// ---- dense operator on differences, as exact digits (deriv_mma.cuh) ----------
+
+namespace {
+
+using real = long double;   // 64 (x86) or 113 (aarch64) bits of mantissa
+static_assert(LDBL_MANT_DIG >= 64, "the entries need 60 exact bits");
+
+// One scheme's rows with exact rational coefficients in `real`
+struct ExactRow {
+    real a, c;           // off-diagonals of A (the diagonal is 1)
+    int first;           // column of the first right-hand-side coefficient
+    real q[7];           // right-hand side: columns first .. first + 6
+};
+
+std::vector<ExactRow> exact_rows(int scheme, int n, bool interior_only) {
+    const bool padeA = scheme == EMIX_SCHEME_A;
+    const real al = padeA ? real(1) / 4 : real(1) / 3, a = padeA ? real(3) / 4 : real(7) / 9,
+               b = padeA ? real(0) : real(1) / 36;
+    std::vector<ExactRow> R(n);
+    for (int i = 0; i < n; ++i) {
+        ExactRow &r = R[i];
+        r.a = r.c = al;
+        r.first = i - 2;
+        const real q[7] = {-b, -a, 0, a, b, 0, 0};
+        for (int k = 0; k < 7; ++k) r.q[k] = q[k];
+    }
+    if (interior_only) return R;
+    const bool b3 = scheme == EMIX_SCHEME_B;
+    const real end[4] = {b3 ? real(-5) / 2 : real(-17) / 6, b3 ? real(2) : real(3) / 2,
+                         b3 ? real(1) / 2 : real(3) / 2, b3 ? real(0) : real(-1) / 6};
+    for (int side = 0; side < 2; ++side) {
+        const int i0 = side ? n - 1 : 0, i1 = side ? n - 2 : 1;
+        const real s = side ? -1 : 1;
+        ExactRow &r = R[i0], &t = R[i1];
+        r.a = side ? (b3 ? 2 : 3) : 0;
+        r.c = side ? 0 : (b3 ? 2 : 3);
+        r.first = side ? n - 7 : 0;
+        for (real &v : r.q) v = 0;
+        for (int k = 0; k < 4; ++k) r.q[side ? 6 - k : k] = s * end[k];
+        t.a = t.c = real(1) / 4;
+        t.first = side ? n - 7 : 0;
+        for (real &v : t.q) v = 0;
+        t.q[side ? 4 : 0] = real(-3) / 4;
+        t.q[side ? 6 : 2] = real(3) / 4;
+    }
+    return R;
+}
+
+// rows of E = (sums over m > k of D_{im}) from the rows of D = A^{-1} B
+class ExactOperator {
+public:
+    ExactOperator(int scheme, int n, bool interior_only) : n_(n), R_(exact_rows(scheme, n, interior_only)), bet_(n), gam_(n + 1) {
+        // A^T: sub-diagonal c_{j-1}, super-diagonal a_{j+1}
+        bet_[0] = 1;
+        for (int j = 1; j < n; ++j) {
+            gam_[j] = R_[j].a / bet_[j - 1];
+            bet_[j] = 1 - R_[j - 1].c * gam_[j];
+        }
+    }
+    // E_{ik} for k in [k0, k0 + cnt); entries beyond reach are added to the ends
+    void row(int i, int k0, int cnt, std::vector<real> &e) const {
+        constexpr int W = 48;   // 0.38^48 = 2^-67
+        const int lo = std::max(0, i - W), hi = std::min(n_ - 1, i + W);
+        std::vector<real> y(hi - lo + 1, real(0));
+        real w = 1 / bet_[i];
+        y[i - lo] = w;
+        for (int j = i + 1; j <= hi; ++j) y[j - lo] = w = -R_[j - 1].c * w / bet_[j];
+        for (int j = hi - 1; j >= lo; --j) y[j - lo] -= gam_[j + 1] * y[j + 1 - lo];
+        const int m0 = lo - 8, m1 = hi + 8;
+        std::vector<real> d(m1 - m0 + 1, real(0));
+        for (int j = lo; j <= hi; ++j)
+            for (int k = 0; k < 7; ++k) {
+                const int m = R_[j].first + k;
+                if (m >= m0 && m <= m1) d[m - m0] += y[j - lo] * R_[j].q[k];
+            }
+        e.assign(cnt, real(0));
+        real s = 0;   // from the right: sum of D_{im}, m > k, for k >= i
+        for (int m = m1; m > i; --m) {
+            s += d[m - m0];
+            e[std::min(std::max(m - 1 - k0, 0), cnt - 1)] += s;
+        }
+        s = 0;        // from the left: minus the sum of D_{im}, m <= k, for k < i
+        for (int m = m0; m < i; ++m) {
+            s += d[m - m0];
+            e[std::min(std::max(m - k0, 0), cnt - 1)] -= s;
+        }
+    }
+
+private:
+    int n_;
+    std::vector<ExactRow> R_;
+    std::vector<real> bet_, gam_;
+};
+
+// an integer of at most 11 bits as f16
+unsigned short half_bits(int v) {
+    if (!v) return 0;
+    const unsigned short sign = v < 0 ? 0x8000 : 0;
+    unsigned m = (unsigned)(v < 0 ? -v : v);
+    int e = 0;
+    while (m >> (e + 1)) ++e;
+    return (unsigned short)(sign | ((e + 15) << 10) | ((m << (10 - e)) & 0x3ff));
+}
+
+// blocks whose rows and differences lie this far from the ends have the
+// interior's entries: the closures' share falls by 0.38 per row on the way
+// to the end and back, 2^-61 here
+constexpr int kMmaEnd = 44;
+
+struct MKey {
+    int dev, scheme, n;
+    double h;
+    bool operator<(const MKey &o) const {
+        return std::tie(dev, scheme, n, h) < std::tie(o.dev, o.scheme, o.n, o.h);
+    }
+};
+std::mutex g_m_mu;
+std::map<MKey, MmaTable> g_m_tables;   // entries and device buffers live until process exit; b null: none
+
+int build_mma(int scheme, int n, double h, double sign, MmaTable &t, std::vector<unsigned short> &b) {
+    const bool per = scheme == EMIX_SCHEME_BPER;
+    t = MmaTable{};
+    t.n = n;
+    t.periodic = per ? 1 : 0;
+    t.nblk = (n + kMmaRows - 1) / kMmaRows;
+    if (per) {
+        t.nlow = t.nhigh = 0;
+        t.ntype = 1;
+    } else {
+        t.nlow = std::min(t.nblk, (kMmaEnd + kMmaRows - 1) / kMmaRows);
+        int first_high = t.nblk;
+        while (first_high > t.nlow && kMmaRows * first_high - 1 > n - 1 - kMmaEnd) --first_high;
+        t.nhigh = t.nblk - first_high;
+        t.ntype = t.nlow + t.nhigh + (first_high > t.nlow ? 1 : 0);
+        if (t.ntype > kMmaMaxTypes) return EMIX_ERR_UNSUPPORTED;
+    }
+    // the interior's rows from a long pencil without closures nearby
+    constexpr int kMid = 160;
+    const ExactOperator inner(scheme, 2 * kMid, true);
+    const ExactOperator own(scheme, per ? 2 * kMid : n, per);
+    constexpr int cnt = kMmaWin * kMmaRows;
+    std::vector<std::vector<real>> E((size_t)t.ntype * kMmaRows);
+    real top = 0;
+    for (int ty = 0; ty < t.ntype; ++ty) {
+        const bool mid = per || (ty == t.nlow && t.ntype > t.nlow + t.nhigh);
+        const int blk = ty < t.nlow ? ty : t.nblk - (t.ntype - ty);
+        for (int o = 0; o < kMmaRows; ++o) {
+            std::vector<real> &e = E[(size_t)ty * kMmaRows + o];
+            if (mid) {
+                inner.row(kMid + o, kMid - 40, cnt, e);
+            } else if (kMmaRows * blk + o < n) {
+                // differences before 0 and after n-2 do not exist; their columns stay zero
+                const int k0 = kMmaRows * blk - 40, ka = std::max(k0, 0), kb = std::min(k0 + cnt, n - 1);
+                std::vector<real> in;
+                own.row(kMmaRows * blk + o, ka, kb - ka, in);
+                e.assign(cnt, real(0));
+                for (int k = ka; k < kb; ++k) e[k - k0] = in[k - ka];
+            } else {
+                e.assign(cnt, real(0));
+            }
+            for (real &v : e) {
+                v *= (real)sign / (real)h;
+                top = std::max(top, std::fabs(v));
+            }
+        }
+    }
+    if (!(top > 0) || !std::isfinite((double)top)) return EMIX_ERR_UNSUPPORTED;
+    const real full = 511 * std::ldexp(real(1), 10 * (kMmaDig - 1));
+    t.se = std::ilogb((double)(full / top));
+    if (std::ldexp(top, t.se) > full) --t.se;
+    b.assign((size_t)t.ntype * kMmaTypeBytes / 2, 0);
+    for (int ty = 0; ty < t.ntype; ++ty) {
+        int lead[kMmaWin];
+        for (int &l : lead) l = kMmaDig;
+        for (int o = 0; o < kMmaRows; ++o) {
+            long size[3] = {0, 0, 0};   // sums of |digit| over the row, per leading digit
+            real sum = 0;
+            for (int k = 0; k < cnt; ++k) {
+                const real v = std::ldexp(E[(size_t)ty * kMmaRows + o][k], t.se);
+                sum += std::fabs(v);
+                long long q = std::llrint((double)std::floor(v / 1073741824.0L));
+                long long r = std::llrint((double)(v - (real)q * 1073741824.0L));   // [0, 2^30]
+                int d[kMmaDig];
+                for (int i = kMmaDig - 1; i >= 0; --i) {
+                    long long &x = i >= 3 ? r : q;
+                    const int dg = (int)((x + 512) & 1023) - 512;
+                    d[i] = dg;
+                    x = (x - dg) / 1024;
+                    if (i == 3) q += r;
+                }
+                const int g = k / kMmaRows, kk = k % kMmaRows;
+                for (int i = 0; i < kMmaDig; ++i) {
+                    if (d[i] && i < lead[g]) lead[g] = i;
+                    if (i < 3) size[i] += std::abs(d[i]);
+                    b[((size_t)ty * kMmaTypeBytes + g * kMmaGroupBytes + (kk / 8) * (kMmaStack * 16) +
+                       (i * kMmaRows + o) * 16) / 2 + kk % 8] = half_bits(d[i]);
+                }
+            }
+            // the f32 sums of the three leading digit orders are exact integers
+            // (the lower orders' worst case, all digits at their bound and of one
+            // sign, exceeds 2^24 by up to 2, costing 2^-48 of the result), and
+            // the combined sum fits 64 bits
+            long s = 0;
+            for (int i = 0; i < 3; ++i) {
+                s += size[i] * 512;
+                if (s >= 1L << 24) return EMIX_ERR_UNSUPPORTED;
+            }
+            if (sum > 4000 * std::ldexp(real(1), 10 * (kMmaDig - 1))) return EMIX_ERR_UNSUPPORTED;
+        }
+        if (std::min(lead[0], lead[kMmaWin - 1]) < kMmaLead0 || std::min(lead[1], lead[kMmaWin - 2]) < kMmaLead1)
+            return EMIX_ERR_UNSUPPORTED;
+    }
+    return EMIX_OK;
+}
+
+} // namespace
+
+int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out) {
+    *out = nullptr;
+    if (n < kMmaMinN) return EMIX_OK;
+    int dev = 0;
+    EMIX_CUDA_TRY(cudaGetDevice(&dev));
+    MKey key{dev, scheme, n, sign * h};
+    std::lock_guard<std::mutex> lock(g_m_mu);
+    auto it = g_m_tables.find(key);
+    if (it == g_m_tables.end()) {
+        MmaTable t{};
+        std::vector<unsigned short> b;
+        if (build_mma(scheme, n, h, sign, t, b)) {
+            t.b = nullptr;
+        } else {
+            void *buf = nullptr;
+            if (cudaMalloc(&buf, b.size() * 2) != cudaSuccess) {
+                cudaGetLastError();
+                set_last_message("cudaMalloc of a tensor-core derivative table failed");
+                return EMIX_ERR_ALLOC;
+            }
+            EMIX_CUDA_TRY(cudaMemcpy(buf, b.data(), b.size() * 2, cudaMemcpyHostToDevice));
+            t.b = (const unsigned short *)buf;
+        }
+        it = g_m_tables.emplace(key, t).first;
+    }
+    if (it->second.b) *out = &it->second;   // map nodes stay where they are
     return EMIX_OK;
 }
 

@@ -11,6 +11,7 @@
 // Only where the rows come from differs.  The reference transposes the field and walks each pencil
 // serially (src/Schemes/derivCompact.cu:8-37,146-215).
 #include "deriv_tma.cuh"
+#include "deriv_mma.cuh"
 #include "tma.cuh"
 
 #include <cstring>
@@ -584,7 +585,10 @@ using namespace emix;
 
 extern "C" int emix_pencil_tma_timeouts(int *count) {
     if (!count) return EMIX_ERR_ARG;
+    int mma = 0;
     EMIX_CUDA_TRY(cudaMemcpyFromSymbol(count, g_pencil_tma_timeouts, sizeof(int)));
+    if (int rc = deriv_mma_timeouts(&mma)) return rc;
+    *count += mma;
     return EMIX_OK;
 }
 

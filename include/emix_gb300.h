@@ -398,20 +398,21 @@ int emix_ctx_tma_stages(emix_ctx *ctx);
  * unwritten; 0 in every correct run. */
 int emix_weno_tma_timeouts(int *count);
 
-/* 1: the flux divergence's y and z passes (the accumulating pencil sweeps)
- * bring the rows they read into shared memory by TMA tiled copies (4 rows x
- * 128 pencils per copy, a ring of three), where the copy unit's rules hold
- * (closed schemes, nx even, 16-byte aligned fields); 0: the threads load
- * them.  The values are the same either way.  emix_ctx_pencil_tma_launches
- * gives how many of the step's launches use the copies.  The reference
+/* 1: the y and z pencil sweeps (divergence, gradients) bring the rows they
+ * read into shared memory by TMA tiled copies (4 rows x 128 pencils per copy,
+ * a ring of three), where the copy unit's rules hold (nx even, 16-byte
+ * aligned fields); 0: the threads load them.  The values are the same either
+ * way.  emix_ctx_pencil_tma_launches gives how many of the step's launches
+ * the rules allow the copies for; axes of 40 rows and more take their
+ * derivatives on the tensor cores instead of a sweep.  The reference
  * transposes each field and walks each pencil serially
  * (src/Schemes/derivCompact.cu:8-37,146-215). */
 int emix_ctx_set_pencil_tma(emix_ctx *ctx, int on);
 int emix_ctx_pencil_tma_launches(emix_ctx *ctx);
 
 /* Pencil blocks (since the library was loaded, on the current device) that
- * gave up waiting for a row copy after about 0.3 s and left their pencils
- * unwritten; 0 in every correct run. */
+ * gave up waiting for a row copy, or for the tensor core, after about 0.3 s
+ * and left their pencils unwritten; 0 in every correct run. */
 int emix_pencil_tma_timeouts(int *count);
 
 /* Test hook for those bounded waits: 1 makes the TMA pencil launches issue
