@@ -251,7 +251,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
     // by up to five blocks at a tile's end; scaled[t]: tile t's (mod 2)
     // magnitudes are in s_part; read[t]: every warp that wants them has them
     __shared__ __align__(8) unsigned long long s_full[2], s_drained[2], s_conv[8], s_done[8],
-        s_scaled[2], s_read[2];
+        s_scaled[2], s_read[2], s_table;
     __shared__ Spread s_part[2][kScanParts][kMmaPencils];   // by the tile's parity
     __shared__ unsigned char s_scalar[kMmaPencils];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -269,19 +269,25 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_conv[q])), "r"(kRoleWarps) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_done[q])) : "memory");
         }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_table)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // the operator's digits, by bulk copies that land during the first scan
+        // (four steps of a 40^3 tank: 1363 us, 1408 with loads before it)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     :: "r"(smem_u32(&s_table)), "r"(M.ntype * kMmaTypeBytes) : "memory");
+        for (int q = 0; q < M.ntype; ++q)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         :: "r"(smem_u32(dyn + q * kMmaTypeBytes)),
+                            "l"(reinterpret_cast<const unsigned char *>(M.b) + (size_t)q * kMmaTypeBytes),
+                            "r"(kMmaTypeBytes), "r"(smem_u32(&s_table)) : "memory");
     }
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_u32(&s_tmem)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    {
-        const uint4 *src = reinterpret_cast<const uint4 *>(M.b);
-        uint4 *dst = reinterpret_cast<uint4 *>(dyn);
-        for (int q = tid; q < M.ntype * (kMmaTypeBytes / 16); q += kMmaThreads) dst[q] = src[q];
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -431,6 +437,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
             const unsigned leader = lane == 0;
             int B = 0, first = 0;     // block, and the tile's first group, counted over the tiles
             int seen = 0;             // groups known to be in tensor memory
+            wait(&s_table, 0);
             for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
                 const Tile jt = tile_of(job, 0);
                 for (int b = jt.b0; b < jt.b1; ++b, ++B) {
