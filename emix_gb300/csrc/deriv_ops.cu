@@ -120,6 +120,37 @@ int launch_deriv_yz_pair(const DerivTable &Ty, const DerivTable &Tz, int nfa, in
 
 namespace {
 
+// Stored x, y and z derivatives of the same fields by the sweeps in one
+// launch of one-warp blocks: x blocks first, then y, then z.  For grids whose
+// axes are all too short for the tensor cores (under 40 rows): each launch is
+// then a fraction of a wave and its time one warp's serial walk, so three in
+// turn cost three walks (24 x 20 x 28, 4 fields: 41 us a call with three
+// launches, 27 with one).
+struct XyzArgs {
+    DerivTable T[3];
+    PencilFields F[3];
+    int nx, ny, nz, xb, yb;   // x and y blocks
+};
+
+__global__ void __launch_bounds__(32) k_deriv_xyz(const __grid_constant__ XyzArgs a) {
+    __shared__ double tile[kXTile];
+    const int nbx = (a.nx + 31) / 32;
+    int b = blockIdx.x;
+    if (b < a.xb) {
+        deriv_x_body<EPI_STORE>(a.T[0], a.F[0], (long)a.ny * a.nz, make_uint3(b, 0, blockIdx.z), threadIdx.x, 1, tile);
+        return;
+    }
+    b -= a.xb;
+    if (b < a.yb) {
+        deriv_yz_body<EPI_STORE>(a.T[1], a.F[1], a.nx, a.nz, (long)a.nx, (long)a.nx * a.ny,
+                                 make_uint3(b % nbx, b / nbx, blockIdx.z), threadIdx.x, 32);
+        return;
+    }
+    b -= a.yb;
+    deriv_yz_body<EPI_STORE>(a.T[2], a.F[2], a.nx, a.ny, (long)a.nx * a.ny, (long)a.nx,
+                             make_uint3(b % nbx, b / nbx, blockIdx.z), threadIdx.x, 32);
+}
+
 bool dims_ok(int nx, int ny, int nz) {
     return nx >= 6 && ny >= 6 && nz >= 6 && nx <= kTableMaxN && ny <= kTableMaxN && nz <= kTableMaxN &&
            ny <= 65535 && nz <= 65535;
@@ -192,14 +223,32 @@ int cudaDeriv_dev_impl(const int schemes[3], double *dvel, double *dtemp, const 
     const size_t n = ncell(nx, ny, nz);
     const int dims[3] = {nx, ny, nz};
     const bool wt = temp != nullptr && dtemp != nullptr;
+    XyzArgs a{};
+    bool sweeps = true;
     for (int ax = 0; ax < 3; ++ax) {
-        DerivTable T;
-        int rc = get_deriv_table(schemes[ax], dims[ax], h[ax], &T);
+        int rc = get_deriv_table(schemes[ax], dims[ax], h[ax], &a.T[ax]);
         if (rc) return rc;
+        sweeps = sweeps && !deriv_on_mma(a.T[ax]);
+        for (int f = 0; f < (wt ? 4 : 3); ++f) {
+            a.F[ax].in[f] = f < 3 ? vel + f * n : temp;
+            a.F[ax].w[f] = a.F[ax].out[f] = f < 3 ? dvel + (3 * ax + f) * n : dtemp + ax * n;
+        }
+    }
+    if (sweeps && nx < kMmaMinN && ny < kMmaMinN && nz < kMmaMinN) {
+        a.nx = nx; a.ny = ny; a.nz = nz;
+        const int nbx = (nx + 31) / 32;
+        a.xb = (ny * nz + 31) / 32;
+        a.yb = nbx * nz;
+        k_deriv_xyz<<<dim3(a.xb + a.yb + nbx * ny, 1, wt ? 4 : 3), 32, 0, st>>>(a);
+        EMIX_CUDA_TRY(cudaGetLastError());
+        return EMIX_OK;
+    }
+    for (int ax = 0; ax < 3; ++ax) {
+        const DerivTable &T = a.T[ax];
         const double *in[4] = {vel, vel + n, vel + 2 * n, temp};
         double *out[4] = {dvel + (3 * ax) * n, dvel + (3 * ax + 1) * n, dvel + (3 * ax + 2) * n,
                           wt ? dtemp + ax * n : nullptr};
-        rc = launch_deriv(T, ax, EPI_STORE, wt ? 4 : 3, in, out, out, nx, ny, nz, st);
+        const int rc = launch_deriv(T, ax, EPI_STORE, wt ? 4 : 3, in, out, out, nx, ny, nz, st);
         if (rc) return rc;
     }
     return EMIX_OK;
