@@ -460,7 +460,9 @@ int emix_cuDivergence(const int schemes[3], double *rs, double *rsv, const doubl
     const double *src[6] = {e, f, g, ev, fv, gv};
     for (int q = 0; q < 6; ++q)
         EMIX_CUDA_TRY(cudaMemcpyAsync(de + q * n, src[q], n * sizeof(double), cudaMemcpyHostToDevice, st));
-    EMIX_CUDA_TRY(cudaMemcpyAsync(dj, jbn, 11 * n * sizeof(double), cudaMemcpyHostToDevice, st));
+    // of the metrics only the five components the divergence reads
+    for (int q : {0, 4, 8, 9, 10})
+        EMIX_CUDA_TRY(cudaMemcpyAsync(dj + q * n, jbn + q * n, n * sizeof(double), cudaMemcpyHostToDevice, st));
     const double h[3] = {hx, hy, hz};
     rc = cuDivergence_dev_impl(schemes, drs, drsv, de, de + n, de + 2 * n, de + 3 * n, de + 4 * n,
                                de + 5 * n, dj, h, nx, ny, nz, st, scr);
