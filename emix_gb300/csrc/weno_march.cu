@@ -5,7 +5,6 @@
 #include "weno_march.cuh"
 
 
-#include <atomic>
 #include <cstring>
 #include <mutex>
 
@@ -22,29 +21,6 @@ __global__ void __launch_bounds__(kNT, 4) k_weno_march_tma(const __grid_constant
     weno_march_body_t<true>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z, &tmap);
 }
 
-
-// resident blocks per SM x SMs of a stage kernel on the current device
-// (queried once per kernel and device ordinal)
-template <class K>
-int resident_blocks(K kernel, std::atomic<int> (&cache)[64]) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-        cudaGetLastError();
-        return device_sms() * 4;
-    }
-    int v = cache[dev].load(std::memory_order_relaxed);
-    if (v > 0) return v;
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kNT, 0) != cudaSuccess) {
-        cudaGetLastError();
-        return device_sms() * 4;
-    }
-    v = device_sms() * (per > 0 ? per : 1);
-    cache[dev].store(v, std::memory_order_relaxed);
-    return v;
-}
-
-std::atomic<int> g_res_plain[64], g_res_tma[64];
 
 } // namespace
 
@@ -84,20 +60,7 @@ bool weno_tma_map(CUtensorMap *m, const WenoArgs &a) {
 int launch_weno_march(const WenoArgs &a, cudaStream_t st, const CUtensorMap *tmap) {
     const int gx = (a.rn[0] + kMX - 1) / kMX, gy = (a.rn[1] + kMY - 1) / kMY;
     if (gy > 65535) return EMIX_ERR_ARG;
-    const int resident = tmap ? resident_blocks(k_weno_march_tma, g_res_tma) : resident_blocks(k_weno_march, g_res_plain);
-    // z chunks: the count whose block total fills the last wave best, chunks
-    // of at least 8 planes, the smaller count on a tie
-    const long cols = (long)gx * gy;
-    long best = 1;
-    double best_eff = 0.0;
-    const long maxgz = a.rn[2] / 8 < 1 ? 1 : (a.rn[2] / 8 > 65535 ? 65535 : a.rn[2] / 8);
-    for (long gz = 1; gz <= maxgz && gz <= 64; ++gz) {
-        const long T = cols * gz;
-        const long waves = (T + resident - 1) / resident;
-        const double eff = (double)T / ((double)waves * resident);
-        if (eff > best_eff + 1e-3) { best_eff = eff; best = gz; }
-    }
-    const dim3 grid(gx, gy, (unsigned)best);
+    const dim3 grid(gx, gy, (unsigned)march_chunks((long)gx * gy, a.rn[2], kMarchStart));
     if (tmap) k_weno_march_tma<<<grid, kNT, 0, st>>>(*tmap, a);
     else k_weno_march<<<grid, kNT, 0, st>>>(a);
     EMIX_CUDA_TRY(cudaGetLastError());
