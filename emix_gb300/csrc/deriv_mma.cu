@@ -26,18 +26,22 @@
 //   eight warps combine the finished block's six sums per output.
 // Whole tiles while they fill every SM, the rest cut into segments of blocks.
 //
-// What bounds it: the roles are within a fifth of one another (per block of
-// 2048 outputs, of about 4300 clocks: instructions issued 2800, conversion
-// 2100 and waits, results 2700, scan 3400 per block's share); the ALU pipe is
-// 54% busy (165 instructions a cell, of which conversion 45, results 30, scan
-// 11 a row), the tensor pipe 15%: an instruction of up to 128 columns takes 80
-// clocks whatever its width, and 16 outputs a block are what tensor memory
-// holds beside the digits.  Measured, ms for 5 fields of 256^3, sweeps -> here:
-// closed x 1.001 -> 0.694, y 0.991 -> 0.577, z 0.991 -> 0.578; cyclic 1.215 ->
-// 0.704, 1.071 -> 0.709, 1.069 -> 0.712; the tank's step at 256^3 34.65 ->
-// 30.36 ms.  Error against a dense solve, 192 x 160 x 192 smooth fields, 2-norm:
-// A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 -> 9.4e-16,
-// C 5.7e-15 -> 3.4e-15.
+// What bounds it: the scanning warps (their loads come from DRAM, 12 KB in
+// flight per SM: a quarter of the scan took y from 0.514 to 0.434 ms) and the
+// tensor-core warp (28 instructions a block at 80 clocks each whatever their
+// width up to 128 columns; 16 outputs a block are what tensor memory holds
+// beside the digits) about alike, with the ALU pipe 55% busy (conversion 45
+// instructions a row, results 30, scan 11).  Two things made the issue of the
+// instructions cheap: elect.sync with warp-uniform operands (0.569 -> 0.522)
+// and a straight run of them, digit by digit, for the blocks whose six groups
+// all exist (-> 0.492).  More or fewer rows a scan step, L2 prefetch of the
+// rows to come, non-allocating loads and the scan spread over the other warps
+// (0.62) measured no better or worse.
+// Measured, ms for 5 fields of 256^3, sweeps -> here: closed x 1.001 -> 0.612,
+// y 0.991 -> 0.492, z 0.991 -> 0.498; cyclic 1.215 -> 0.557, 1.071 -> 0.588,
+// 1.069 -> 0.592.  Error against a dense solve, 192 x 160 x 192 smooth fields,
+// 2-norm: A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 ->
+// 9.4e-16, C 5.7e-15 -> 3.4e-15.
 //
 // Pencils with infinities or NaN, or of magnitudes whose fixed-point
 // exponents would leave the FP64 range, take the scalar sweep (deriv.cuh)
@@ -131,12 +135,11 @@ EMIX_DEV unsigned digit_pair(unsigned a, unsigned b) {
     return *reinterpret_cast<const unsigned *>(&h);
 }
 
-// digit P of a thread's rows to tensor memory
+// digit P of a thread's rows as pairs of f16
 template <int P>
-EMIX_DEV void put_digits(unsigned addr, const unsigned (&w)[kRpt]) {
-    static_assert(kRpt == 8, "one x4 store per digit");
-    tm_st4(addr, digit_pair<P>(w[0], w[1]), digit_pair<P>(w[2], w[3]), digit_pair<P>(w[4], w[5]),
-           digit_pair<P>(w[6], w[7]));
+EMIX_DEV void digits(unsigned (&d)[kRpt / 2], const unsigned (&w)[kRpt]) {
+#pragma unroll
+    for (int q = 0; q < kRpt / 2; ++q) d[q] = digit_pair<P>(w[2 * q], w[2 * q + 1]);
 }
 
 // one pencil's magnitudes, once known: the exponent its values are fixed to,
@@ -254,7 +257,10 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
         s_scaled[2], s_read[2], s_table;
     __shared__ Spread s_part[2][kScanParts][kMmaPencils];   // by the tile's parity
     __shared__ unsigned char s_scalar[kMmaPencils];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
+    // through a shuffle: the roles' branches are then known to be uniform, and
+    // the instruction operands stay in uniform registers
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int n = T.n;
 
     if (tid == 0) {
@@ -434,7 +440,8 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
     if (warp == 2 * kRoleWarps) {
         // ---- the tensor core's warp ----------------------------------------
         {
-            const unsigned leader = lane == 0;
+            unsigned leader;
+            asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
             int B = 0, first = 0;     // block, and the tile's first group, counted over the tiles
             int seen = 0;             // groups known to be in tensor memory
             wait(&s_table, 0);
@@ -455,22 +462,40 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
                         (1ull << 46) | ((unsigned long long)(128 >> 4) << 32) |
                         ((unsigned long long)((kMmaStack * 16) >> 4) << 16);
                     const unsigned sums = tm + (unsigned)(B & 1) * kAccCols;
+                    constexpr int kLead[kMmaWin] = {kMmaLead0, kMmaLead1, 0, 0, kMmaLead1, kMmaLead0};
+                    // the group in window place w: its digits' columns and operand
+                    unsigned ah[kMmaWin], al[kMmaWin], lo[kMmaWin];
 #pragma unroll
-                    for (int q = 0; q < kMmaWin; ++q) {
-                        const int w = q == 0 ? 2 : (q <= 2 ? q - 1 : q);   // the block's own group first
-                        constexpr int kLead[kMmaWin] = {kMmaLead0, kMmaLead1, 0, 0, kMmaLead1, kMmaLead0};
-                        const int lead = kLead[w], g = b - 2 + w;
-                        if (g < jt.ga || g > jt.gb) continue;
-                        const unsigned c = (unsigned)(first + g - jt.ga);
-                        const unsigned ah = tm + kHighCol + (c % kHighRing) * 24, al = tm + kLowCol + (c % kLowRing) * 24;
-                        const unsigned bb = base + w * kMmaGroupBytes + lead * (kMmaRows * 16);
-                        const unsigned long long desc = desc0 | ((bb >> 4) & 0x3fff);
+                    for (int w = 0; w < kMmaWin; ++w) {
+                        const unsigned c = (unsigned)(first + b - 2 + w - jt.ga + kHighRing * kLowRing);
+                        ah[w] = tm + kHighCol + (c % kHighRing) * 24;
+                        al[w] = tm + kLowCol + (c % kLowRing) * 24;
+                        lo[w] = ((base + w * kMmaGroupBytes + kLead[w] * (kMmaRows * 16)) >> 4) & 0x3fff;
+                    }
+                    // digit j of the group in place w; the block's own group (w = 2)
+                    // comes first and sets every sum
+                    auto product = [&](int w, int j) {
+                        const unsigned idesc = (1u << 4) | ((unsigned)((kMmaDig - kLead[w] - j) * kMmaRows >> 3) << 17) |
+                                               ((kMmaPencils >> 4) << 24);
+                        mma_f16(sums + (kLead[w] + j) * kMmaRows, j < 3 ? ah[w] + j * 8 : al[w] + (j - 3) * 8,
+                                desc0 | lo[w], idesc, !(w == 2 && j == 0), leader);
+                    };
+                    constexpr int kOrder[kMmaWin] = {2, 0, 1, 3, 4, 5};
+                    if (b - 2 >= jt.ga && b + 3 <= jt.gb) {
+                        // digit by digit: instructions on the same sums follow one
+                        // another (1900 clocks a block alone, 2180 group by group)
 #pragma unroll
-                        for (int j = 0; j < kMmaDig - lead; ++j) {
-                            const unsigned idesc = (1u << 4) | ((unsigned)((kMmaDig - lead - j) * kMmaRows >> 3) << 17) |
-                                                   ((kMmaPencils >> 4) << 24);
-                            mma_f16(sums + (lead + j) * kMmaRows, j < 3 ? ah + j * 8 : al + (j - 3) * 8, desc, idesc,
-                                    !(q == 0 && j == 0), leader);
+                        for (int j = 0; j < kMmaDig; ++j)
+#pragma unroll
+                            for (int q = 0; q < kMmaWin; ++q)
+                                if (j < kMmaDig - kLead[kOrder[q]]) product(kOrder[q], j);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < kMmaWin; ++q) {
+                            const int w = kOrder[q], g = b - 2 + w;
+                            if (g < jt.ga || g > jt.gb) continue;
+#pragma unroll
+                            for (int j = 0; j < kMmaDig - kLead[w]; ++j) product(w, j);
                         }
                     }
                     __syncwarp();
@@ -544,6 +569,8 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
                 for (int q = 0; q < kRpt; ++q) t[((rtid >> 4) + (kRole / 16) * q) * kXPitch + (rtid & 15)] = v[q];
                 if (rtid < kMmaPencils) t[rtid * kXPitch + 16] = v[kRpt];
             };
+            // the staged rows' (x: tile c's) digits
+            unsigned dg[kMmaDig][kRpt / 2];
             auto convert = [&](int c, const Scale &sc) {
                 unsigned w1[kRpt], w2[kRpt];
                 const double *t = xin + (c & 1) * kXTileDoubles + slot_p * kXPitch + kRpt * rg;
@@ -557,19 +584,23 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
                     w1[q] = (unsigned)(y >> 32);
                     w2[q] = (unsigned)(y >> 4);
                 }
+                digits<22>(dg[0], w1);
+                digits<12>(dg[1], w1);
+                digits<2>(dg[2], w1);
+                digits<20>(dg[3], w2);
+                digits<10>(dg[4], w2);
+                digits<0>(dg[5], w2);
+            };
+            auto put = [&](int c) {
                 const unsigned ah = tml + kHighCol + (unsigned)(c % kHighRing) * 24 + rg * (kRpt / 2);
                 const unsigned al = tml + kLowCol + (unsigned)(c % kLowRing) * 24 + rg * (kRpt / 2);
-                put_digits<22>(ah, w1);
-                put_digits<12>(ah + 8, w1);
-                put_digits<2>(ah + 16, w1);
-                put_digits<20>(al, w2);
-                put_digits<10>(al + 8, w2);
-                put_digits<0>(al + 16, w2);
+#pragma unroll
+                for (int j = 0; j < kMmaDig; ++j)
+                    tm_st4((j < 3 ? ah : al) + j % 3 * 8, dg[j][0], dg[j][1], dg[j][2], dg[j][3]);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 arrive(&s_conv[c & 7]);
             };
-
             int c = 0, done = 0, t = 0, B = 0;   // groups, finished blocks, jobs, the job's first block
             int job = blockIdx.x;
             Tile cur = tile_of(job, slot_p), last = cur;
@@ -599,13 +630,15 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
                         if (k + 1 < ng) load(cur, cur.ga + k + 1);
                         else if (more) load(nxt, nxt.ga);
                     }
-                    for (; done <= need; ++done) wait(&s_done[done & 7], (unsigned)(done >> 3) & 1);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    // the arithmetic first, so that only the stores wait for the blocks
                     convert(c, sc);
                     if constexpr (!XAX) {
                         if (k + 1 < ng) load(cur, cur.ga + k + 1);
                         else if (more) load(nxt, nxt.ga);
                     }
+                    for (; done <= need; ++done) wait(&s_done[done & 7], (unsigned)(done >> 3) & 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    put(c);
                 }
                 B += cur.b1 - cur.b0;
                 last = cur;
