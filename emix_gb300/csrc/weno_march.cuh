@@ -109,27 +109,21 @@ EMIX_DEV void weno_z_general(const double *phi, long id, int Z, int nzg, bool le
     }
 }
 
-// z chunks of a marching launch over `cols` columns of nz planes.  The FP64
-// pipe bounds the march (256 cells of a plane keep an SM busy for 16,000
-// clocks), so an SM's time is the planes it gets however they are divided
-// between its blocks: the chunk length whose most loaded SM has the fewest
-// planes, a chunk's start (the window of differences, the first copies)
-// counted as kMarchStart planes.  Against chunks of at least 8 planes that fill
-// the last wave of resident blocks: four steps of a 40^3 tank (16 columns on
-// 152 SMs) 2.06 -> 1.90 ms, the 160 x 160 x 128 host-buffer step 7.49 -> 7.31,
-// the 256^3 step 30.36 -> 30.22; 0.03 to 0.14 measure alike, 0 and 0.6 lose up
-// to 5%.
-constexpr double kMarchStart = 0.1;
-inline int march_chunks(long cols, int nz, double start) {
-    const long sms = device_sms();
-    double best = 0.0;
-    int gz = 1;
-    for (int c = 1; c <= nz; ++c) {
-        const int k = (nz + c - 1) / c;
-        const double t = (double)((cols * k + sms - 1) / sms) * (c + start);
-        if (k <= 65535 && (best == 0.0 || t < best)) { best = t; gz = k; }
-    }
-    return gz;
+// z chunks of a marching launch over `cols` columns of nz planes.  Short
+// chunks pay their start (the window of differences, the first copies: a tenth
+// of a plane) more often, long ones leave SMs idle behind the most loaded one
+// (a quarter of a chunk on average: blocks land unevenly, and a lone block is
+// no faster per plane than four).  With P planes per SM the sum of both,
+// 0.1 P / c + c / 4, is least at c = sqrt(P / 2.5).  Lengths of 1 to 64 planes
+// measured: 40^3 1 (0.138 ms a step, 12 planes 0.355), 64^3 1-2 (0.318), 96^3
+// 4 (0.822, this rule 0.831, one block per SM 1.05), 128^3 5 (1.710), 160 x 160
+// x 128 6 (2.569); the reinitialisation's stages alike (96^3 3, 130 x 118 x 106
+// 5).
+inline int march_chunks(long cols, int nz) {
+    const double planes = (double)cols * nz / device_sms();
+    int c = (int)(sqrt(planes / 2.5) + 0.5);
+    if (c < nz / 65535 + 1) c = nz / 65535 + 1;
+    return (nz + c - 1) / c;
 }
 
 struct Plane {
