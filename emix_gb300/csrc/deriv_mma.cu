@@ -51,6 +51,9 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <vector>
+
 namespace emix {
 namespace {
 
@@ -240,11 +243,14 @@ EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, i
 
 // XAX: pencils along x (rows contiguous, brought through a shared tile);
 // otherwise along y or z (pencils contiguous along x)
+// CTA `cta` of the I.ncta that share the item
 template <bool XAX, int EPI, bool PER>
-__global__ void __launch_bounds__(kMmaThreads, 1)
-k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTable M,
-            const __grid_constant__ PencilFields F, int np, int ntile, int nf, int whole, int segs, int nx,
-            long s, long os) {
+EMIX_DEV void mma_body(const MmaItem &I, int cta) {
+    const DerivTable &T = I.T;
+    const MmaTable &M = I.M;
+    const PencilFields &F = I.F;
+    const int np = I.np, ntile = I.ntile, nf = I.nf, whole = I.whole, segs = I.segs, nx = I.nx, ncta = I.ncta;
+    const long s = I.s, os = I.os;
     extern __shared__ __align__(1024) unsigned char dyn[];
     __shared__ unsigned s_tmem;
     __shared__ int s_fail;
@@ -433,7 +439,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
     constexpr int kPencilWarps = 2 * kRoleWarps + kScanWarps;   // all but the tensor core's
     if (warp != 2 * kRoleWarps) {
         // the first tile's, by all of them
-        scan_tile(blockIdx.x, 0, warp < 2 * kRoleWarps ? warp : warp - 1, kPencilWarps);
+        scan_tile(cta, 0, warp < 2 * kRoleWarps ? warp : warp - 1, kPencilWarps);
         asm volatile("bar.sync 3, %0;" :: "n"(32 * kPencilWarps) : "memory");
     }
 
@@ -445,7 +451,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
             int B = 0, first = 0;     // block, and the tile's first group, counted over the tiles
             int seen = 0;             // groups known to be in tensor memory
             wait(&s_table, 0);
-            for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
+            for (int job = cta; job < jobs; job += ncta) {
                 const Tile jt = tile_of(job, 0);
                 for (int b = jt.b0; b < jt.b1; ++b, ++B) {
                     for (const int need = first + min(b + 3, jt.gb) - jt.ga; seen <= need; ++seen)
@@ -510,7 +516,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
     } else if (warp > 2 * kRoleWarps) {
         // ---- magnitudes of the tiles' pencils, one tile ahead ------------------
         int t = 1;
-        for (int job = blockIdx.x + gridDim.x; job < jobs; job += gridDim.x, ++t) {
+        for (int job = cta + ncta; job < jobs; job += ncta, ++t) {
             if (t >= 2) wait(&s_read[t & 1], (unsigned)((t - 2) >> 1) & 1);   // s_part's turn
             scan_tile(job, t & 1, warp - 2 * kRoleWarps - 1, kScanWarps);
             arrive(&s_scaled[t & 1]);
@@ -602,7 +608,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
                 arrive(&s_conv[c & 7]);
             };
             int c = 0, done = 0, t = 0, B = 0;   // groups, finished blocks, jobs, the job's first block
-            int job = blockIdx.x;
+            int job = cta;
             Tile cur = tile_of(job, slot_p), last = cur;
             // the last block (counted over the jobs) that reads group `pos` of a
             // job, `reach` groups behind it at most; of one before the previous
@@ -615,11 +621,11 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
                 return pos >= 0 ? Bl + min(last.ga + pos + reach, last.b1 - 1) - last.b0 : Bl - 1;
             };
             load(cur, cur.ga);
-            for (; job < jobs; job += gridDim.x, ++t) {
+            for (; job < jobs; job += ncta, ++t) {
                 const Scale sc = scale_wait(t);
-                const bool more = job + (int)gridDim.x < jobs;
+                const bool more = job + ncta < jobs;
                 Tile nxt = cur;
-                if (more) nxt = tile_of(job + gridDim.x, slot_p);
+                if (more) nxt = tile_of(job + ncta, slot_p);
                 const int ng = cur.gb - cur.ga + 1;
                 for (int k = 0; k < ng; ++k, ++c) {
                     // the rings' places are free once the blocks that read them are done
@@ -662,7 +668,7 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
 
             // ---- the stream of blocks ----------------------------------------------
             int B = 0, t = 0;
-            for (int job = blockIdx.x; job < jobs; job += gridDim.x, ++t) {
+            for (int job = cta; job < jobs; job += ncta, ++t) {
                 const Tile cur = tile_of(job, slot_p);
                 const Scale sc = scale_wait(t);
                 const int escale = (sc.E - 1023 - M.se - sc.sh) * (1 << 20);
@@ -749,43 +755,122 @@ k_deriv_mma(const __grid_constant__ DerivTable T, const __grid_constant__ MmaTab
 }
 
 template <bool XAX, int EPI, bool PER>
-int launch(const DerivTable &T, const MmaTable &M, const PencilFields &F, int nf, int np, int nx, long s, long os,
-           cudaStream_t st) {
-    // tensor memory is taken whole: at least 116 KB of shared memory keeps a
-    // second CTA off the SM
-    size_t shm = (size_t)M.ntype * kMmaTypeBytes + (XAX ? 4 * kXTileDoubles * sizeof(double) : 0);
-    if (shm < 120 * 1024) shm = 120 * 1024;
-    auto kernel = k_deriv_mma<XAX, EPI, PER>;
-    EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-    const int ntile = (np + kMmaPencils - 1) / kMmaPencils, tiles = ntile * nf, sms = device_sms();
-    // whole tiles while they fill every SM; what is left is cut into the
-    // number of segments (each with five more groups to convert) that ends
-    // first
-    const int whole = tiles / sms * sms, rest = tiles - whole;
-    int segs = 1;
-    long best = -1;
-    for (int c = 1; rest > 0 && c <= M.nblk && c <= 64; ++c) {
-        const long rounds = ((long)rest * c + sms - 1) / sms, t = rounds * ((M.nblk + c - 1) / c + 6);
-        if (best < 0 || t < best) { best = t; segs = c; }
+__global__ void __launch_bounds__(kMmaThreads, 1) k_deriv_mma(const __grid_constant__ MmaItem I) {
+    mma_body<XAX, EPI, PER>(I, blockIdx.x);
+}
+
+// many grids' derivatives: the SMs are divided between the items (mma_split)
+template <bool XAX, int EPI, bool PER>
+__global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaItem *__restrict__ items, int count) {
+    __shared__ MmaItem s_item;
+    int g = 0;
+    for (int hi = count - 1; g < hi;) {
+        const int mid = (g + hi + 1) >> 1;
+        if (items[mid].cta0 <= (int)blockIdx.x) g = mid; else hi = mid - 1;
     }
-    const long jobs = whole + (long)rest * segs;
-    const int grid = (int)(jobs < sms ? jobs : sms);
-    kernel<<<grid, kMmaThreads, shm, st>>>(T, M, F, np, ntile, nf, whole, segs, nx, s, os);
+    static_assert(sizeof(MmaItem) % sizeof(int) == 0, "copied by words");
+    for (int q = threadIdx.x; q < (int)(sizeof(MmaItem) / sizeof(int)); q += kMmaThreads)
+        reinterpret_cast<int *>(&s_item)[q] = reinterpret_cast<const int *>(items + g)[q];
+    __syncthreads();
+    mma_body<XAX, EPI, PER>(s_item, (int)blockIdx.x - s_item.cta0);
+}
+
+// tensor memory is taken whole: at least 116 KB of shared memory keeps a
+// second CTA off the SM
+template <bool XAX>
+int shared_bytes(int ntype) {
+    const int shm = ntype * kMmaTypeBytes + (XAX ? 4 * kXTileDoubles * (int)sizeof(double) : 0);
+    return shm < 120 * 1024 ? 120 * 1024 : shm;
+}
+
+// divides item I between at most `n` CTAs (I.ncta: those that get work):
+// whole tiles while they fill every CTA; what is left is cut into the number
+// of segments (each with five more groups to convert) that ends first.
+// Returns the blocks and starts the most loaded CTA walks
+long divide(MmaItem &I, int n) {
+    const int tiles = I.ntile * I.nf, rest = tiles % n;
+    I.whole = tiles - rest;
+    I.segs = 1;
+    long best = 0;
+    for (int c = 1; rest > 0 && c <= I.M.nblk && c <= 64; ++c) {
+        const long rounds = ((long)rest * c + n - 1) / n, t = rounds * ((I.M.nblk + c - 1) / c + 6);
+        if (c == 1 || t < best) { best = t; I.segs = c; }
+    }
+    const long jobs = I.whole + (long)rest * I.segs;
+    I.ncta = (int)(jobs < n ? jobs : n);
+    return best + (long)(I.whole / n) * (I.M.nblk + 6);
+}
+
+template <bool XAX, int EPI, bool PER>
+int launch(const MmaItem &I, cudaStream_t st) {
+    const int shm = shared_bytes<XAX>(I.M.ntype);
+    auto kernel = k_deriv_mma<XAX, EPI, PER>;
+    EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+    kernel<<<I.ncta, kMmaThreads, shm, st>>>(I);
     EMIX_CUDA_TRY(cudaGetLastError());
     return EMIX_OK;
 }
 
-template <bool XAX>
-int launch(int epi, const DerivTable &T, const MmaTable &M, const PencilFields &F, int nf, int np, int nx, long s,
-           long os, cudaStream_t st) {
-    if (M.periodic)
-        return epi == EPI_STORE ? launch<XAX, EPI_STORE, true>(T, M, F, nf, np, nx, s, os, st)
-                                : launch<XAX, EPI_ACCUM, true>(T, M, F, nf, np, nx, s, os, st);
-    return epi == EPI_STORE ? launch<XAX, EPI_STORE, false>(T, M, F, nf, np, nx, s, os, st)
-                            : launch<XAX, EPI_ACCUM, false>(T, M, F, nf, np, nx, s, os, st);
+template <bool XAX, int EPI, bool PER>
+int launch(const MmaBatch &b, cudaStream_t st) {
+    const int shm = shared_bytes<XAX>(b.ntype);
+    auto kernel = k_batch_deriv_mma<XAX, EPI, PER>;
+    EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+    kernel<<<b.ctas, kMmaThreads, shm, st>>>(b.items, b.count);
+    EMIX_CUDA_TRY(cudaGetLastError());
+    return EMIX_OK;
+}
+
+// the variant for an item or a batch of items
+template <class W>
+int launch_variant(bool xax, int epi, bool per, const W &w, cudaStream_t st) {
+    if (xax) {
+        if (per) return epi == EPI_STORE ? launch<true, EPI_STORE, true>(w, st) : launch<true, EPI_ACCUM, true>(w, st);
+        return epi == EPI_STORE ? launch<true, EPI_STORE, false>(w, st) : launch<true, EPI_ACCUM, false>(w, st);
+    }
+    if (per) return epi == EPI_STORE ? launch<false, EPI_STORE, true>(w, st) : launch<false, EPI_ACCUM, true>(w, st);
+    return epi == EPI_STORE ? launch<false, EPI_STORE, false>(w, st) : launch<false, EPI_ACCUM, false>(w, st);
 }
 
 } // namespace
+
+MmaItem mma_item(const DerivTable &T, const MmaTable &M, int axis, const PencilFields &F, int nf, int nx, int ny,
+                 int nz) {
+    MmaItem I{};
+    I.T = T;
+    I.M = M;
+    I.F = F;
+    I.nf = nf;
+    I.nx = nx;
+    I.np = axis == 0 ? ny * nz : nx * (axis == 1 ? nz : ny);
+    I.s = axis == 0 ? 1 : (axis == 1 ? (long)nx : (long)nx * ny);
+    I.os = axis == 0 ? 0 : (axis == 1 ? (long)nx * ny : (long)nx);
+    I.ntile = (I.np + kMmaPencils - 1) / kMmaPencils;
+    return I;
+}
+
+MmaBatch mma_split(MmaItem *items, int count) {
+    // one CTA each, then one at a time to the item that would end last
+    const int sms = device_sms();
+    std::vector<int> n(count, 1);
+    std::vector<long> t(count);
+    for (int g = 0; g < count; ++g) t[g] = divide(items[g], 1);
+    for (int left = sms - count; left > 0; --left) {
+        const int g = (int)(std::max_element(t.begin(), t.end()) - t.begin());
+        t[g] = divide(items[g], ++n[g]);
+    }
+    MmaBatch b{nullptr, count, 0, 0};
+    for (int g = 0; g < count; ++g) {
+        items[g].cta0 = b.ctas;
+        b.ctas += items[g].ncta;
+        b.ntype = std::max(b.ntype, items[g].M.ntype);
+    }
+    return b;
+}
+
+int launch_deriv_mma_batch(const MmaBatch &b, bool xax, int epi, bool periodic, cudaStream_t st) {
+    return launch_variant(xax, epi, periodic, b, st);
+}
 
 int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
                      double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st) {
@@ -795,10 +880,9 @@ int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, 
         F.w[f] = w[f];
         F.out[f] = out[f];
     }
-    const int nother = axis == 0 ? 0 : (axis == 1 ? nz : ny);
-    if (axis == 0) return launch<true>(epi, T, M, F, nf, ny * nz, nx, 1, 0, st);
-    const long s = axis == 1 ? (long)nx : (long)nx * ny, os = axis == 1 ? (long)nx * ny : (long)nx;
-    return launch<false>(epi, T, M, F, nf, nx * nother, nx, s, os, st);
+    MmaItem I = mma_item(T, M, axis, F, nf, nx, ny, nz);
+    divide(I, device_sms());
+    return launch_variant(axis == 0, epi, M.periodic != 0, I, st);
 }
 
 int deriv_mma_timeouts(int *count) {

@@ -66,6 +66,29 @@ inline bool deriv_on_mma(const DerivTable &T) { return T.mma != nullptr; }
 int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
                      double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st);
 
+// One derivative of nf fields of a grid, and the CTAs that walk its tiles.
+struct MmaItem {
+    DerivTable T;
+    MmaTable M;
+    PencilFields F;
+    int np, ntile, nf, nx;    // pencils, tiles of them, fields
+    int whole, segs;          // whole tiles, and segments each of the others is cut into
+    int cta0, ncta;           // CTAs [cta0, cta0 + ncta) of the launch
+    long s, os;               // strides along a pencil, and between lines of pencils
+};
+MmaItem mma_item(const DerivTable &T, const MmaTable &M, int axis, const PencilFields &F, int nf, int nx, int ny,
+                 int nz);
+
+// Many items (all along x or none, all cyclic or none) as one launch.
+struct MmaBatch {
+    const MmaItem *items;     // on the device
+    int count, ctas, ntype;   // items, CTAs of the launch, most block types of a table
+};
+// divides the SMs between the items, by their work (an item is at least one
+// CTA); `items` of the result is left to the caller
+MmaBatch mma_split(MmaItem *items, int count);
+int launch_deriv_mma_batch(const MmaBatch &b, bool xax, int epi, bool periodic, cudaStream_t st);
+
 // blocks that gave up a bounded wait since the library was loaded
 int deriv_mma_timeouts(int *count);
 
