@@ -108,6 +108,11 @@ __global__ void __launch_bounds__(256, 2) k_smag_flux(SmagArgs s, FluxArgs f) {
 __global__ void k_sgs_sf(SfArgs a) { EMIX_FOR_CELLS(q, a.n) sf_cell(a, q); }
 __global__ void k_vort(VortArgs a) { EMIX_FOR_CELLS(q, a.n) vort_cell(a, q); }
 __global__ void k_selective(SelArgs a) { EMIX_FOR_CELLS(q, a.n) select_cell(a, q); }
+// 17 to 23 FP64 operations and 21 to 26 fields a cell: the FP64 pipe bounds it.
+// Its blocks take different times (the impeller's cells), so there are 64 a
+// SM, not the resident 8.  256^3, three launches with their walls: 3.50 ms ->
+// 2.90 (64-bit indices and unscaled sums 3.50, 8 blocks a SM 3.19, one block
+// per 256 cells 3.05).
 __global__ void k_rk_post(RkArgs a) {
     const long end = a.qend > 0 ? a.qend : rk_count(a);
     for (long q = a.qbeg + blockIdx.x * (long)blockDim.x + threadIdx.x; q < end; q += (long)gridDim.x * blockDim.x)

@@ -280,11 +280,17 @@ __host__ __device__ inline long rk_count(const RkArgs &a) {
     return (a.walls && a.faces) ? rk_face_count(a.nx, a.ny, a.nz) : a.n;
 }
 
-// RK3 combination of one cell (rungek_ico.f90:89-90, 153-154, 217-220)
-EMIX_DEV void rk_combine(const RkArgs &a, long q, double v[5]) {
+// RK3 combination of one cell (rungek_ico.f90:89-90, 153-154, 217-220), up to
+// the factor rk_scale: um0 + dt R; 3 um0 + um + dt R (of 1/4);
+// um0 + 2 um + 2 dt R (of 1/3).  The FP64 pipe bounds the update, and the
+// factor cancels in the velocities, so it is left to the density and the last
+// equation (27 -> 23 FP64 operations a cell).
+EMIX_DEV double rk_scale(int stage) { return stage == 1 ? 1.0 : (stage == 2 ? 0.25 : 1.0 / 3.0); }
+
+EMIX_DEV void rk_sums(const RkArgs &a, long q, double v[5]) {
     const long n = a.n;
     // the substep's weight of dt*R times the metric factor jbn(11), once per cell
-    const double w = a.stage == 1 ? a.dt : (a.stage == 2 ? 0.25 * a.dt : (2.0 / 3.0) * a.dt);
+    const double w = a.stage == 3 ? 2.0 * a.dt : a.dt;
     const double cj = w * a.jbn[10 * n + q];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
@@ -293,11 +299,19 @@ EMIX_DEV void rk_combine(const RkArgs &a, long q, double v[5]) {
         if (a.stage == 1)
             b = u0;
         else if (a.stage == 2)
-            b = fma(0.25, a.um[m * n + q], 0.75 * u0);
+            b = fma(3.0, u0, a.um[m * n + q]);
         else
-            b = fma(2.0 / 3.0, a.um[m * n + q], (1.0 / 3.0) * u0);
+            b = fma(2.0, a.um[m * n + q], u0);
         v[m] = fma(cj, a.R[m * n + q], b);
     }
+}
+
+EMIX_DEV void rk_combine(const RkArgs &a, long q, double v[5]) {
+    rk_sums(a, q, v);
+    if (a.stage == 1) return;
+    const double c = rk_scale(a.stage);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) v[m] *= c;
 }
 
 // fmax(-6, fmin(6, x)) by integer compares on the bit pattern (|x| > 6 takes
@@ -310,14 +324,22 @@ EMIX_DEV double clip6(double x) {
 }
 
 // varc_to_varnc + clip + mask + varc_to_varnc (:104-124), then the rebuild
-// after the level-set call site (:127-138), of the combined values v
-EMIX_DEV void rk_convert(const RkArgs &a, long q, double v[5]) {
+// after the level-set call site (:127-138), of the combined values v c
+EMIX_DEV void rk_convert(const RkArgs &a, long q, double v[5], double c) {
     const long n = a.n;
+    double pc = a.inv_m2 * c;
     if (a.imp.on && a.impflag[q]) {
         // rushton(stage) after the walls (rungek_ico.f90:102); cells the
         // impeller cannot reach are left as they are
+        double f[5];   // of its own: its address is taken
+#pragma unroll
+        for (int m = 0; m < 5; ++m) f[m] = v[m] * c;
+        c = 1.0;
+        pc = a.inv_m2;
         impeller_force_cell(a.imp, a.clock + 2 + 2 * (a.stage - 1) * kImpMaxBlades, a.xyz[q],
-                            a.xyz[n + q], a.xyz[2 * n + q], v, nullptr);
+                            a.xyz[n + q], a.xyz[2 * n + q], f, nullptr);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) v[m] = f[m];
     }
     const double r = v[0];
     const double rr = rcp_fast(r);
@@ -337,7 +359,7 @@ EMIX_DEV void rk_convert(const RkArgs &a, long q, double v[5]) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) uu[d] = clip6(v[d + 1] * rr) * mk;
     }
-    const double p = r * a.inv_m2;
+    const double p = r * pc;
     const double r1 = p * (a.mach * a.mach);
     a.out[q] = r1;
 #pragma unroll
@@ -345,7 +367,7 @@ EMIX_DEV void rk_convert(const RkArgs &a, long q, double v[5]) {
         a.out[(d + 1) * n + q] = uu[d] * r1;
         a.u[d * n + q] = uu[d];
     }
-    a.out[4 * n + q] = v[4];
+    a.out[4 * n + q] = a.stage == 1 ? v[4] : v[4] * c;
     a.pres[q] = p;
 }
 
@@ -380,44 +402,54 @@ EMIX_DEV void wall_x(const RkArgs &a, int i, int j, int k, double v[5]) {
 EMIX_DEV void rk_cell(const RkArgs &a, long q) {
     double v[5];
     if (!a.walls) {
-        rk_combine(a, q, v);
-        rk_convert(a, q, v);
+        rk_sums(a, q, v);
+        rk_convert(a, q, v, rk_scale(a.stage));
         return;
     }
-    const int nx = a.nx, ny = a.ny, nz = a.nz;
-    int i, j, k;
+    // 32-bit indices (a context of 2^32 cells does not fit in memory): the
+    // conversions of 64-bit divisions run at the FP64 pipe's rate
+    const unsigned nx = a.nx, ny = a.ny, nz = a.nz;
+    unsigned i, j, k, r = (unsigned)q;
     if (!a.faces) {
-        i = (int)(q % nx);
-        j = (int)((q / nx) % ny);
-        k = (int)(q / ((long)nx * ny));
+        const unsigned row = r / nx;
+        k = row / ny;
+        j = row - k * ny;
+        i = r - row * nx;
         if (i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || k == 0 || k >= nz - 2) return;
-        rk_combine(a, q, v);
-        rk_convert(a, q, v);
+        rk_sums(a, q, v);
+        rk_convert(a, q, v, rk_scale(a.stage));
         return;
     }
-    const long pz = (long)nx * ny, py = (long)nx * (nz - 3);
-    if (q < 3 * pz) {
-        const int pl = (int)(q / pz);
-        const long r = q - pl * pz;
-        i = (int)(r % nx); j = (int)(r / nx); k = pl == 0 ? 0 : nz - 3 + pl;
-    } else if (q < 3 * pz + 2 * py) {
-        const long r0 = q - 3 * pz;
-        const int pl = (int)(r0 / py);
-        const long r = r0 - pl * py;
-        i = (int)(r % nx); k = 1 + (int)(r / nx); j = pl == 0 ? 0 : ny - 1;
+    const unsigned pz = nx * ny, py = nx * (nz - 3), px = (ny - 2) * (nz - 3);
+    if (r < 3 * pz) {
+        const unsigned pl = r / pz;
+        r -= pl * pz;
+        j = r / nx;
+        i = r - j * nx;
+        k = pl == 0 ? 0 : nz - 3 + pl;
+    } else if (r < 3 * pz + 2 * py) {
+        r -= 3 * pz;
+        const unsigned pl = r / py;
+        r -= pl * py;
+        k = r / nx;
+        i = r - k * nx;
+        ++k;
+        j = pl == 0 ? 0 : ny - 1;
     } else {
-        const long px = (long)(ny - 2) * (nz - 3);
-        const long r0 = q - 3 * pz - 2 * py;
-        const int pl = (int)(r0 / px);
-        const long r = r0 - pl * px;
-        j = 1 + (int)(r % (ny - 2)); k = 1 + (int)(r / (ny - 2)); i = pl == 0 ? 0 : nx - 1;
+        r -= 3 * pz + 2 * py;
+        const unsigned pl = r / px;
+        r -= pl * px;
+        k = r / (ny - 2);
+        j = 1 + r - k * (ny - 2);
+        ++k;
+        i = pl == 0 ? 0 : nx - 1;
     }
     // the wall rules read only cells no rule writes (k = 1, nz-3; j = 1,
     // ny-2; i = 1, nx-2 after the earlier rules), recomputed here from the RK
     // inputs, which this launch does not overwrite: it runs before the launch
     // over the other cells, and writes only wall cells
     wall_x(a, i, j, k, v);
-    rk_convert(a, i + (long)nx * (j + (long)ny * k), v);
+    rk_convert(a, i + (long)nx * (j + (long)ny * k), v, 1.0);
 }
 
 // ---- kernels ------------------------------------------------------------------

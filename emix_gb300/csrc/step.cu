@@ -40,7 +40,7 @@ __global__ void k_metric_products(const double *__restrict__ jbn, double *__rest
 int launch_single(const Launch &L, cudaStream_t st) {
     switch (L.kind) {
     case LK_PRIM:
-        k_prim<<<cells_grid(L.prim.n), 256, 0, st>>>(L.prim);
+        k_prim<<<grid_cap(L.prim.n, 64), 256, 0, st>>>(L.prim);
         break;
     case LK_PAD:
         k_ghost_pad<<<cells_grid(L.pad.qend > 0 ? L.pad.qend - L.pad.qbeg : L.pad.ng), 256, 0, st>>>(L.pad);
@@ -71,7 +71,7 @@ int launch_single(const Launch &L, cudaStream_t st) {
         k_flux_all<<<cells_grid(L.flux.n), 256, 0, st>>>(L.flux);
         break;
     case LK_RK:
-        k_rk_post<<<cells_grid(rk_count(L.rk)), 256, 0, st>>>(L.rk);
+        k_rk_post<<<grid_cap(rk_count(L.rk), 64), 256, 0, st>>>(L.rk);
         break;
     case LK_BC:
         k_bc<<<cells_grid(bc_count(L.bc)), 256, 0, st>>>(L.bc);
