@@ -58,7 +58,7 @@ struct VortOp { using A = VortArgs; static EMIX_DEV void cell(const A &a, long q
 struct SelOp { using A = SelArgs; static EMIX_DEV void cell(const A &a, long q) { select_cell(a, q); } static EMIX_DEV long cnt(const A &a) { return a.n; } };
 struct FluxOp { using A = FluxArgs; static EMIX_DEV void cell(const A &a, long q) { flux_cell(a, q); } static EMIX_DEV long cnt(const A &a) { return a.n; } };
 struct BcOp { using A = BcArgs; static EMIX_DEV void cell(const A &a, long q) { bc_cell(a, q); } static EMIX_DEV long cnt(const A &a) { return bc_count(a); } };
-struct ClockOp { using A = ImpClockArgs; static EMIX_DEV void cell(const A &a, long q) { if (q == 0) imp_clock_tick(a); } static EMIX_DEV long cnt(const A &) { return 1; } };
+struct ClockOp { using A = ImpClockArgs; static EMIX_DEV void cell(const A &a, long q) { imp_clock_tick(a, (int)q); } static EMIX_DEV long cnt(const A &) { return 32; } };
 struct RkOp { using A = RkArgs; static EMIX_DEV void cell(const A &a, long q) { rk_cell(a, q); } static EMIX_DEV long cnt(const A &a) { return rk_count(a); } };
 
 template <class Op>
@@ -285,7 +285,7 @@ long point_count(const Launch &L) {
     case LK_FLUX: return L.flux.n;
     case LK_RK: return rk_count(L.rk);
     case LK_BC: return bc_count(L.bc);
-    case LK_CLOCK: return 1;
+    case LK_CLOCK: return 32;   // one warp
     default: return 0;
     }
 }

@@ -5,7 +5,7 @@
 namespace emix {
 
 __global__ void k_imp_clock(ImpClockArgs a) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) imp_clock_tick(a);
+    imp_clock_tick(a, threadIdx.x);   // one warp
 }
 
 __global__ void k_imp_flags(const double *xyz, ImpGeom g, long n, unsigned char *flag) {

@@ -331,7 +331,7 @@ EMIX_DEV void rk_convert(const RkArgs &a, long q, double v[5], double c) {
     if (a.imp.on && a.impflag[q]) {
         // rushton(stage) after the walls (rungek_ico.f90:102); cells the
         // impeller cannot reach are left as they are
-        double f[5];   // of its own: its address is taken
+        double f[5];
 #pragma unroll
         for (int m = 0; m < 5; ++m) f[m] = v[m] * c;
         c = 1.0;
