@@ -38,8 +38,8 @@
 // rows to come, non-allocating loads and the scan spread over the other warps
 // (0.62) measured no better or worse.
 // Measured, ms for 5 fields of 256^3, sweeps -> here: closed x 1.001 -> 0.612,
-// y 0.991 -> 0.492, z 0.991 -> 0.498; cyclic 1.215 -> 0.557, 1.071 -> 0.588,
-// 1.069 -> 0.592.  Error against a dense solve, 192 x 160 x 192 smooth fields,
+// y 0.991 -> 0.492, z 0.991 -> 0.498; cyclic 1.215 -> 0.557, 1.071 -> 0.567,
+// 1.069 -> 0.571.  Error against a dense solve, 192 x 160 x 192 smooth fields,
 // 2-norm: A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 ->
 // 9.4e-16, C 5.7e-15 -> 3.4e-15.
 //
@@ -551,7 +551,17 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             // ---- a group's rows to digits, loaded one group ahead ---------------
             double v[kRpt + 1];   // y, z: the thread's rows; x: staged values
             auto load = [&](const Tile &t, int g) {
-                const int k = kMmaRows * g - 8;
+                int k = kMmaRows * g - 8;
+                if constexpr (PER) {
+                    // once for the group; its rows then wrap at most once (a loop
+                    // for each: 5 fields of 64^3 31 us, here 25; 128^3 105, 91)
+                    while (k < 0) k += n;
+                    while (k >= n) k -= n;
+                }
+                auto wrap = [&](int r) {
+                    if constexpr (PER) return r >= n ? r - n : r;
+                    return min(max(r, 0), n - 1);
+                };
                 if constexpr (!XAX) {
                     if (k >= 0 && k + kMmaRows < n) {
                         const double *fp = t.in + (long)(k + kRpt * rg) * s;
@@ -559,14 +569,14 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                         for (int q = 0; q <= kRpt; ++q) v[q] = fp[q * s];
                     } else {
 #pragma unroll
-                        for (int q = 0; q <= kRpt; ++q) v[q] = t.in[(long)row_of(k + kRpt * rg + q) * s];
+                        for (int q = 0; q <= kRpt; ++q) v[q] = t.in[(long)wrap(k + kRpt * rg + q) * s];
                     }
                 } else {
-                    const int row = row_of(k + (rtid & 15));
+                    const int row = wrap(k + (rtid & 15));
 #pragma unroll
                     for (int q = 0; q < kRpt; ++q)
                         v[q] = t.in[(long)min(t.p0 + (rtid >> 4) + (kRole / 16) * q, np - 1) * n + row];
-                    if (rtid < kMmaPencils) v[kRpt] = t.in[(long)min(t.p0 + rtid, np - 1) * n + row_of(k + 16)];
+                    if (rtid < kMmaPencils) v[kRpt] = t.in[(long)min(t.p0 + rtid, np - 1) * n + wrap(k + 16)];
                 }
             };
             auto stage = [&](int c) {   // x: into the tile of group c
