@@ -52,6 +52,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 namespace emix {
@@ -75,6 +76,18 @@ constexpr int kAccCols = kMmaDig * kMmaRows;
 constexpr int kHighRing = 7, kLowRing = 6;
 constexpr int kHighCol = 2 * kAccCols, kLowCol = kHighCol + kHighRing * 24;
 constexpr int kTmemCols = 512;
+// Kinds of pencils: closed, cyclic, and short cyclic ones of whole groups, all of
+// whose groups are held in tensor memory at once and read round the cycle by the
+// blocks, instead of five of them converted twice.  At least three groups (which
+// wrap once) and at most four (which leave two places for the next tile's).  5
+// fields of 64^3, us: x 28.2 -> 22.6, y and z 25.1 -> 20.7.  A kind of its own:
+// tested at run time it costs the other cyclic pencils 2% (256^3 562 -> 574).
+constexpr int kClosed = 0, kCyclic = 1, kRound = 2;
+constexpr int kMmaRoundN = 64;
+static_assert(kMmaMinN > 2 * kMmaRows && kMmaRoundN / kMmaRows < kLowRing, "kMmaRoundN");
+int kind_of(int n, bool periodic) {
+    return !periodic ? kClosed : (n % kMmaRows == 0 && n <= kMmaRoundN ? kRound : kCyclic);
+}
 constexpr int kMmaWaitNs = 10000, kMmaWaitLimit = 1 << 15;   // a wait's slices, and their number
 constexpr int kXPitch = 17;                 // x pencils' staging tile: 17 rows, odd pitch
 constexpr int kXTileDoubles = kMmaPencils * kXPitch;
@@ -178,7 +191,7 @@ struct Tile {
 
 // magnitudes of the 128 x pencils from p0 of field f: P at a time, lanes along
 // the rows, kScan / P rounds of 32 rows each (P = 1: as many as it takes)
-template <int P, bool PER>
+template <int P, int PER>
 EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, int lane, Spread *to) {
     constexpr int C = kScan / P;
     const int steps = P == 1 ? (n + 32 * C - 1) / (32 * C) : 1;
@@ -244,7 +257,7 @@ EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, i
 // XAX: pencils along x (rows contiguous, brought through a shared tile);
 // otherwise along y or z (pencils contiguous along x)
 // CTA `cta` of the I.ncta that share the item
-template <bool XAX, int EPI, bool PER>
+template <bool XAX, int EPI, int PER>
 EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     const DerivTable &T = I.T;
     const MmaTable &M = I.M;
@@ -311,6 +324,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     const int g0 = PER ? -2 : 0;                                   // first and last group of a tile
     const int g1 = PER ? nblk + 2 : (n + 6) / kMmaRows;
     const int jobs = whole + (ntile * nf - whole) * segs;
+    constexpr bool round = PER == kRound;
     bool ok = true;                                                // false: a wait ran out; nothing is stored any more
 
     // bounded wait; once one has run out no further one is waited for, and
@@ -357,8 +371,8 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         }
         t.b0 = nblk * seg / cut;
         t.b1 = nblk * (seg + 1) / cut;
-        t.ga = max(g0, t.b0 - 2);
-        t.gb = min(g1, t.b1 + 2);
+        t.ga = round ? 0 : max(g0, t.b0 - 2);
+        t.gb = round ? nblk - 1 : min(g1, t.b1 + 2);
         t.field = id / ntile;
         t.p0 = (id - t.field * ntile) * kMmaPencils;
         const int p = min(t.p0 + slot_p, np - 1);
@@ -473,7 +487,9 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                     unsigned ah[kMmaWin], al[kMmaWin], lo[kMmaWin];
 #pragma unroll
                     for (int w = 0; w < kMmaWin; ++w) {
-                        const unsigned c = (unsigned)(first + b - 2 + w - jt.ga + kHighRing * kLowRing);
+                        int g = b - 2 + w;
+                        if (round) g += g < 0 ? nblk : (g >= nblk ? -nblk : 0);
+                        const unsigned c = (unsigned)(first + g - jt.ga + kHighRing * kLowRing);
                         ah[w] = tm + kHighCol + (c % kHighRing) * 24;
                         al[w] = tm + kLowCol + (c % kLowRing) * 24;
                         lo[w] = ((base + w * kMmaGroupBytes + kLead[w] * (kMmaRows * 16)) >> 4) & 0x3fff;
@@ -487,7 +503,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                                 desc0 | lo[w], idesc, !(w == 2 && j == 0), leader);
                     };
                     constexpr int kOrder[kMmaWin] = {2, 0, 1, 3, 4, 5};
-                    if (b - 2 >= jt.ga && b + 3 <= jt.gb) {
+                    if (round || (b - 2 >= jt.ga && b + 3 <= jt.gb)) {
                         // digit by digit: instructions on the same sums follow one
                         // another (1900 clocks a block alone, 2180 group by group)
 #pragma unroll
@@ -624,6 +640,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             // job, `reach` groups behind it at most; of one before the previous
             // job, the last of that
             auto last_use = [&](int pos, int reach) {
+                if (round) reach = nblk;
                 if (pos >= 0) return B + min(cur.ga + pos + reach, cur.b1 - 1) - cur.b0;
                 const int Bl = B - (last.b1 - last.b0);
                 if (t == 0) return -1;
@@ -764,13 +781,13 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(kTmemCols));
 }
 
-template <bool XAX, int EPI, bool PER>
+template <bool XAX, int EPI, int PER>
 __global__ void __launch_bounds__(kMmaThreads, 1) k_deriv_mma(const __grid_constant__ MmaItem I) {
     mma_body<XAX, EPI, PER>(I, blockIdx.x);
 }
 
 // many grids' derivatives: the SMs are divided between the items (mma_split)
-template <bool XAX, int EPI, bool PER>
+template <bool XAX, int EPI, int PER>
 __global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaItem *__restrict__ items, int count) {
     __shared__ MmaItem s_item;
     int g = 0;
@@ -811,7 +828,7 @@ long divide(MmaItem &I, int n) {
     return best + (long)(I.whole / n) * (I.M.nblk + 6);
 }
 
-template <bool XAX, int EPI, bool PER>
+template <bool XAX, int EPI, int PER>
 int launch(const MmaItem &I, cudaStream_t st) {
     const int shm = shared_bytes<XAX>(I.M.ntype);
     auto kernel = k_deriv_mma<XAX, EPI, PER>;
@@ -821,7 +838,7 @@ int launch(const MmaItem &I, cudaStream_t st) {
     return EMIX_OK;
 }
 
-template <bool XAX, int EPI, bool PER>
+template <bool XAX, int EPI, int PER>
 int launch(const MmaBatch &b, cudaStream_t st) {
     const int shm = shared_bytes<XAX>(b.ntype);
     auto kernel = k_batch_deriv_mma<XAX, EPI, PER>;
@@ -832,14 +849,17 @@ int launch(const MmaBatch &b, cudaStream_t st) {
 }
 
 // the variant for an item or a batch of items
+template <bool XAX, int EPI, class W>
+int launch_kind(int kind, const W &w, cudaStream_t st) {
+    if constexpr (std::is_same<W, MmaItem>::value)   // (a batch's launch holds pencils of all lengths)
+        if (kind == kRound) return launch<XAX, EPI, kRound>(w, st);
+    return kind == kCyclic ? launch<XAX, EPI, kCyclic>(w, st) : launch<XAX, EPI, kClosed>(w, st);
+}
+
 template <class W>
-int launch_variant(bool xax, int epi, bool per, const W &w, cudaStream_t st) {
-    if (xax) {
-        if (per) return epi == EPI_STORE ? launch<true, EPI_STORE, true>(w, st) : launch<true, EPI_ACCUM, true>(w, st);
-        return epi == EPI_STORE ? launch<true, EPI_STORE, false>(w, st) : launch<true, EPI_ACCUM, false>(w, st);
-    }
-    if (per) return epi == EPI_STORE ? launch<false, EPI_STORE, true>(w, st) : launch<false, EPI_ACCUM, true>(w, st);
-    return epi == EPI_STORE ? launch<false, EPI_STORE, false>(w, st) : launch<false, EPI_ACCUM, false>(w, st);
+int launch_variant(bool xax, int epi, int kind, const W &w, cudaStream_t st) {
+    if (xax) return epi == EPI_STORE ? launch_kind<true, EPI_STORE>(kind, w, st) : launch_kind<true, EPI_ACCUM>(kind, w, st);
+    return epi == EPI_STORE ? launch_kind<false, EPI_STORE>(kind, w, st) : launch_kind<false, EPI_ACCUM>(kind, w, st);
 }
 
 } // namespace
@@ -879,7 +899,7 @@ MmaBatch mma_split(MmaItem *items, int count) {
 }
 
 int launch_deriv_mma_batch(const MmaBatch &b, bool xax, int epi, bool periodic, cudaStream_t st) {
-    return launch_variant(xax, epi, periodic, b, st);
+    return launch_variant(xax, epi, periodic ? kCyclic : kClosed, b, st);
 }
 
 int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
@@ -892,7 +912,7 @@ int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, 
     }
     MmaItem I = mma_item(T, M, axis, F, nf, nx, ny, nz);
     divide(I, device_sms());
-    return launch_variant(axis == 0, epi, M.periodic != 0, I, st);
+    return launch_variant(axis == 0, epi, kind_of(T.n, M.periodic != 0), I, st);
 }
 
 int deriv_mma_timeouts(int *count) {

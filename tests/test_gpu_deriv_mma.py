@@ -108,3 +108,16 @@ def test_the_same_bits_however_tiles_are_cut(emix, axis):
     for k in (0, 4):
         one = emix.deriv_dev(_dev(f[k]), axis, 0.01, F.SCHEME_C).cpu().numpy()
         assert np.array_equal(many[k], one)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("n, others", [(48, (170, 130)), (64, (170, 130)), (64, (9, 10)), (80, (90, 130))])
+def test_short_cyclic_pencils_of_whole_groups(emix, oracle, axis, n, others):
+    """Cyclic pencils of whole groups of 16, held at once up to 64 rows: several
+    tiles a CTA (and the cut ones), few pencils, and the length above."""
+    dims = list(others)
+    dims.insert(2 - axis, n)   # (nz, ny, nx)
+    f = np.stack([_field(tuple(dims), 7), _field(tuple(dims), 8)])
+    got = emix.deriv_dev(_dev(f), axis, 1.0 / n, F.SCHEME_BPER).cpu().numpy()
+    for c in range(2):
+        assert_close(got[c], oracle.deriv3d(F.SCHEME_BPER, axis, f[c], 1.0 / n), what=f"axis {axis} n {n} field {c}")
