@@ -71,7 +71,8 @@ __global__ void __launch_bounds__(256) k_adj_rk_a(RkAdjArgs A) {
         const long q = q0 + threadIdx.x;
         if (q < n) {
             double v[5];
-            const int i = (int)(q % nx), j = (int)((q / nx) % ny), k = (int)(q / ((long)nx * ny));
+            int i, j, k;
+            cell_of(q, n, nx, ny, i, j, k);
             if (a.walls && (i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || k == 0 || k >= nz - 2))
                 wall_x(a, i, j, k, v);
             else

@@ -43,6 +43,22 @@ inline int grid_cap(long n, int per_sm, int bs = 256) {
     return (int)(b < 1 ? 1 : b);
 }
 
+// (i, j, k) of cell q of an nx x ny x .. grid of n cells.  In 32 bits where the
+// cells' number allows it: a 64-bit division converts on the FP64 pipe (three of
+// them 4 of its operations a cell).
+EMIX_DEV void cell_of(long q, long n, int nx, int ny, int &i, int &j, int &k) {
+    if (n <= 0xffffffffL) {
+        const unsigned r = (unsigned)q, row = r / (unsigned)nx, pl = row / (unsigned)ny;
+        i = (int)(r - row * (unsigned)nx);
+        j = (int)(row - pl * (unsigned)ny);
+        k = (int)pl;
+    } else {
+        i = (int)(q % nx);
+        j = (int)((q / nx) % ny);
+        k = (int)(q / ((long)nx * ny));
+    }
+}
+
 // Per-axis factor table of one compact first-derivative operator, built on
 // the host by build_deriv_table() and read by the pencil kernels.
 //

@@ -164,9 +164,8 @@ EMIX_DEV void sf_cell(const SfArgs &a, long q) {
     const double *U = a.u, *V = a.u + n, *W = a.u + 2 * n;
     const double *ratios = a.ratios;
     const long sy = nx, sz = (long)nx * ny;
-    const int i = (int)(q % nx);
-    const int j = (int)((q / nx) % ny);
-    const int k = (int)(q / sz);
+    int i, j, k;
+    cell_of(q, n, nx, ny, i, j, k);
     double x, y, z, s;
     long p, m;
     // the six one-sided increments in the order of f_structura
@@ -228,9 +227,8 @@ EMIX_DEV void select_cell(const SelArgs &a, long q) {
     const long n = a.n;
     const double *wx = a.w, *wy = a.w + n, *wz = a.w + 2 * n;
     const long sy = nx, sz = (long)nx * ny;
-    const int i = (int)(q % nx);
-    const int j = (int)((q / nx) % ny);
-    const int k = (int)(q / sz);
+    int i, j, k;
+    cell_of(q, n, nx, ny, i, j, k);
     const long a1 = i < nx - 1 ? q + 1 : q, a2 = i > 0 ? q - 1 : q;
     const long a3 = k < nz - 1 ? q + sz : q, a4 = k > 0 ? q - sz : q;
     const long a5 = j < ny - 1 ? q + sy : q, a6 = j > 0 ? q - sy : q;

@@ -147,9 +147,8 @@ EMIX_DEV int mirror(int G, int g, int n) {
 EMIX_DEV void pad_cell(const PadArgs &a, long q) {
     const int g = a.g, nx = a.nx, ny = a.ny, nz = a.nz;
     const int nxg = nx + 2 * g, nyg = ny + 2 * g;
-    const int X = (int)(q % nxg);
-    const int Y = (int)((q / nxg) % nyg);
-    const int Z = (int)(q / ((long)nxg * nyg));
+    int X, Y, Z;
+    cell_of(q, a.ng, nxg, nyg, X, Y, Z);
     const int cnt = (X < g || X >= nx + g) + (Y < g || Y >= ny + g) + (Z < g || Z >= nz + g);
     double v = a.val[mirror(X, g, nx) + (long)nx * (mirror(Y, g, ny) + (long)ny * mirror(Z, g, nz))];
     for (int c = 0; c < cnt; ++c) v *= a.dir;
