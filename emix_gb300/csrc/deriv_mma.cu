@@ -43,6 +43,12 @@
 // 2-norm: A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 ->
 // 9.4e-16, C 5.7e-15 -> 3.4e-15.
 //
+// D^T of the closed schemes (the adjoint) is a table of the same form and one
+// FP64 operation more on the ends' rows: the gradient of a 96^3 tank objective
+// over three steps 18.7 -> 16.9 ms; error against a dense transpose no larger
+// than the sweeps' (192 rows: A 8.0e-16 -> 5.4e-16, B 4.0e-16 -> 3.2e-16, C
+// 8.4e-16 -> 6.2e-16).
+//
 // Pencils with infinities or NaN, or of magnitudes whose fixed-point
 // exponents would leave the FP64 range, take the scalar sweep (deriv.cuh)
 // after the tile.
@@ -76,13 +82,13 @@ constexpr int kAccCols = kMmaDig * kMmaRows;
 constexpr int kHighRing = 7, kLowRing = 6;
 constexpr int kHighCol = 2 * kAccCols, kLowCol = kHighCol + kHighRing * 24;
 constexpr int kTmemCols = 512;
-// Kinds of pencils: closed, cyclic, and short cyclic ones of whole groups, all of
+// Kinds of pencils: closed, closed under D^T, cyclic, and short cyclic ones of whole groups, all of
 // whose groups are held in tensor memory at once and read round the cycle by the
 // blocks, instead of five of them converted twice.  At least three groups (which
 // wrap once) and at most four (which leave two places for the next tile's).  5
 // fields of 64^3, us: x 28.2 -> 22.6, y and z 25.1 -> 20.7.  A kind of its own:
 // tested at run time it costs the other cyclic pencils 2% (256^3 562 -> 574).
-constexpr int kClosed = 0, kCyclic = 1, kRound = 2;
+constexpr int kClosed = 0, kCyclic = 1, kRound = 2, kTransposed = 3;
 constexpr int kMmaRoundN = 64;
 static_assert(kMmaMinN > 2 * kMmaRows && kMmaRoundN / kMmaRows < kLowRing, "kMmaRoundN");
 int kind_of(int n, bool periodic) {
@@ -191,7 +197,7 @@ struct Tile {
 
 // magnitudes of the 128 x pencils from p0 of field f: P at a time, lanes along
 // the rows, kScan / P rounds of 32 rows each (P = 1: as many as it takes)
-template <int P, int PER>
+template <int P, bool PER>
 EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, int lane, Spread *to) {
     constexpr int C = kScan / P;
     const int steps = P == 1 ? (n + 32 * C - 1) / (32 * C) : 1;
@@ -257,9 +263,9 @@ EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, i
 // XAX: pencils along x (rows contiguous, brought through a shared tile);
 // otherwise along y or z (pencils contiguous along x)
 // CTA `cta` of the I.ncta that share the item
-template <bool XAX, int EPI, int PER>
+template <bool XAX, int EPI, int KIND>
 EMIX_DEV void mma_body(const MmaItem &I, int cta) {
-    const DerivTable &T = I.T;
+    constexpr bool PER = KIND == kCyclic || KIND == kRound;
     const MmaTable &M = I.M;
     const PencilFields &F = I.F;
     const int np = I.np, ntile = I.ntile, nf = I.nf, whole = I.whole, segs = I.segs, nx = I.nx, ncta = I.ncta;
@@ -280,7 +286,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     // through a shuffle: the roles' branches are then known to be uniform, and
     // the instruction operands stay in uniform registers
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int n = T.n;
+    const int n = M.n;
 
     if (tid == 0) {
         s_fail = 0;
@@ -324,7 +330,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     const int g0 = PER ? -2 : 0;                                   // first and last group of a tile
     const int g1 = PER ? nblk + 2 : (n + 6) / kMmaRows;
     const int jobs = whole + (ntile * nf - whole) * segs;
-    constexpr bool round = PER == kRound;
+    constexpr bool round = KIND == kRound;
     bool ok = true;                                                // false: a wait ran out; nothing is stored any more
 
     // bounded wait; once one has run out no further one is waited for, and
@@ -724,7 +730,17 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                     if constexpr (!XAX) {
                         if (cur.live && !sc.scalar && ok) {
                             double *o = cur.out + (long)row * s;
-                            if (row + kRpt <= n) {
+                            if (KIND == kTransposed && (b < M.nlow || b >= nblk - M.nhigh)) {
+                                // the ends' blocks: the row sums' share
+#pragma unroll
+                                for (int q = 0; q < kRpt; ++q) {
+                                    if (row + q >= n) break;
+                                    const long at = (long)(row + q) * s;
+                                    double r = fma(M.sigma[row + q], cur.in[at], combine(acc, q, escale));
+                                    if constexpr (EPI == EPI_ACCUM) r += old[q];
+                                    cur.out[at] = r;
+                                }
+                            } else if (row + kRpt <= n) {
 #pragma unroll
                                 for (int q = 0; q < kRpt; ++q) {
                                     double r = combine(acc, q, escale);
@@ -753,6 +769,8 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                             const int pp = (rtid >> 4) + (kRole / 16) * q;
                             if (frow < n && cur.p0 + pp < np && !s_scalar[pp] && ok) {
                                 double r = tl[pp * kXPitch + (rtid & 15)];
+                                if (KIND == kTransposed && (b < M.nlow || b >= nblk - M.nhigh))
+                                    r = fma(M.sigma[frow], cur.in[(long)(cur.p0 + pp) * n + frow], r);
                                 if (EPI == EPI_ACCUM) r += *o;
                                 *o = r;
                             }
@@ -763,7 +781,11 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                 // the pencils outside the fixed-point range
                 if (rg == 0 && sc.scalar && cur.live && ok && cur.b0 == 0) {
                     const long x = XAX ? cur.wofs : 0;
-                    deriv_pencil<EPI>(T, cur.in + x, pick(F.w, cur.field) + cur.wofs, cur.out + x, s);
+                    double *w = pick(F.w, cur.field) + cur.wofs;
+                    if constexpr (KIND == kTransposed)
+                        deriv_t_pencil<EPI == EPI_ACCUM>(I.TT, cur.in + x, w, cur.out + x, s);
+                    else
+                        deriv_pencil<EPI>(I.T, cur.in + x, w, cur.out + x, s);
                 }
                 if constexpr (XAX) row_sync(2);   // s_scalar is free
             }
@@ -781,13 +803,13 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(kTmemCols));
 }
 
-template <bool XAX, int EPI, int PER>
+template <bool XAX, int EPI, int KIND>
 __global__ void __launch_bounds__(kMmaThreads, 1) k_deriv_mma(const __grid_constant__ MmaItem I) {
-    mma_body<XAX, EPI, PER>(I, blockIdx.x);
+    mma_body<XAX, EPI, KIND>(I, blockIdx.x);
 }
 
 // many grids' derivatives: the SMs are divided between the items (mma_split)
-template <bool XAX, int EPI, int PER>
+template <bool XAX, int EPI, int KIND>
 __global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaItem *__restrict__ items, int count) {
     __shared__ MmaItem s_item;
     int g = 0;
@@ -799,7 +821,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaIte
     for (int q = threadIdx.x; q < (int)(sizeof(MmaItem) / sizeof(int)); q += kMmaThreads)
         reinterpret_cast<int *>(&s_item)[q] = reinterpret_cast<const int *>(items + g)[q];
     __syncthreads();
-    mma_body<XAX, EPI, PER>(s_item, (int)blockIdx.x - s_item.cta0);
+    mma_body<XAX, EPI, KIND>(s_item, (int)blockIdx.x - s_item.cta0);
 }
 
 // tensor memory is taken whole: at least 116 KB of shared memory keeps a
@@ -828,20 +850,20 @@ long divide(MmaItem &I, int n) {
     return best + (long)(I.whole / n) * (I.M.nblk + 6);
 }
 
-template <bool XAX, int EPI, int PER>
+template <bool XAX, int EPI, int KIND>
 int launch(const MmaItem &I, cudaStream_t st) {
     const int shm = shared_bytes<XAX>(I.M.ntype);
-    auto kernel = k_deriv_mma<XAX, EPI, PER>;
+    auto kernel = k_deriv_mma<XAX, EPI, KIND>;
     EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     kernel<<<I.ncta, kMmaThreads, shm, st>>>(I);
     EMIX_CUDA_TRY(cudaGetLastError());
     return EMIX_OK;
 }
 
-template <bool XAX, int EPI, int PER>
+template <bool XAX, int EPI, int KIND>
 int launch(const MmaBatch &b, cudaStream_t st) {
     const int shm = shared_bytes<XAX>(b.ntype);
-    auto kernel = k_batch_deriv_mma<XAX, EPI, PER>;
+    auto kernel = k_batch_deriv_mma<XAX, EPI, KIND>;
     EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     kernel<<<b.ctas, kMmaThreads, shm, st>>>(b.items, b.count);
     EMIX_CUDA_TRY(cudaGetLastError());
@@ -851,8 +873,10 @@ int launch(const MmaBatch &b, cudaStream_t st) {
 // the variant for an item or a batch of items
 template <bool XAX, int EPI, class W>
 int launch_kind(int kind, const W &w, cudaStream_t st) {
-    if constexpr (std::is_same<W, MmaItem>::value)   // (a batch's launch holds pencils of all lengths)
+    if constexpr (std::is_same<W, MmaItem>::value) {   // (a batch holds pencils of all lengths, of D)
         if (kind == kRound) return launch<XAX, EPI, kRound>(w, st);
+        if (kind == kTransposed) return launch<XAX, EPI, kTransposed>(w, st);
+    }
     return kind == kCyclic ? launch<XAX, EPI, kCyclic>(w, st) : launch<XAX, EPI, kClosed>(w, st);
 }
 
@@ -902,17 +926,29 @@ int launch_deriv_mma_batch(const MmaBatch &b, bool xax, int epi, bool periodic, 
     return launch_variant(xax, epi, periodic ? kCyclic : kClosed, b, st);
 }
 
-int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
-                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st) {
+static PencilFields fields_of(int nf, const double *const *in, double *const *w, double *const *out) {
     PencilFields F{};
     for (int f = 0; f < nf; ++f) {
         F.in[f] = in[f];
         F.w[f] = w[f];
         F.out[f] = out[f];
     }
-    MmaItem I = mma_item(T, M, axis, F, nf, nx, ny, nz);
+    return F;
+}
+
+int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
+                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st) {
+    MmaItem I = mma_item(T, M, axis, fields_of(nf, in, w, out), nf, nx, ny, nz);
     divide(I, device_sms());
     return launch_variant(axis == 0, epi, kind_of(T.n, M.periodic != 0), I, st);
+}
+
+int launch_deriv_t_mma(const DerivTTable &T, int axis, int acc, int nf, const double *const *in, double *const *w,
+                       double *const *out, int nx, int ny, int nz, cudaStream_t st) {
+    MmaItem I = mma_item(DerivTable{}, *T.mma, axis, fields_of(nf, in, w, out), nf, nx, ny, nz);
+    I.TT = T;
+    divide(I, device_sms());
+    return launch_variant(axis == 0, acc ? EPI_ACCUM : EPI_STORE, kTransposed, I, st);
 }
 
 int deriv_mma_timeouts(int *count) {
