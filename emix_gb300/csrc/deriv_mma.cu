@@ -37,7 +37,7 @@
 // all exist (-> 0.492).  More or fewer rows a scan step, L2 prefetch of the
 // rows to come, non-allocating loads and the scan spread over the other warps
 // (0.62) measured no better or worse.
-// Measured, ms for 5 fields of 256^3, sweeps -> here: closed x 1.001 -> 0.612,
+// Measured, ms for 5 fields of 256^3, sweeps -> here: closed x 1.001 -> 0.537,
 // y 0.991 -> 0.492, z 0.991 -> 0.498; cyclic 1.215 -> 0.557, 1.071 -> 0.567,
 // 1.069 -> 0.571.  Error against a dense solve, 192 x 160 x 192 smooth fields,
 // 2-norm: A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 ->
@@ -91,6 +91,10 @@ constexpr int kTmemCols = 512;
 constexpr int kClosed = 0, kCyclic = 1, kRound = 2, kTransposed = 3;
 constexpr int kMmaRoundN = 64;
 static_assert(kMmaMinN > 2 * kMmaRows && kMmaRoundN / kMmaRows < kLowRing, "kMmaRoundN");
+// x: tiles of finished blocks.  A closed table's seven block types leave 28 KB of
+// L1 beside two of them, 60 KB beside one, and what is in flight lives there: 5
+// fields of 256^3 0.610 ms with two, 0.537 with one and another barrier a block.
+constexpr int out_tiles(int kind) { return kind == kClosed || kind == kTransposed ? 1 : 2; }
 int kind_of(int n, bool periodic) {
     return !periodic ? kClosed : (n % kMmaRows == 0 && n <= kMmaRoundN ? kRound : kCyclic);
 }
@@ -331,6 +335,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     const int g1 = PER ? nblk + 2 : (n + 6) / kMmaRows;
     const int jobs = whole + (ntile * nf - whole) * segs;
     constexpr bool round = KIND == kRound;
+    constexpr int kOutTiles = out_tiles(KIND);
     bool ok = true;                                                // false: a wait ran out; nothing is stored any more
 
     // bounded wait; once one has run out no further one is waited for, and
@@ -757,7 +762,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                             }
                         }
                     } else {
-                        double *tl = xout + (B & 1) * kXTileDoubles;
+                        double *tl = xout + (kOutTiles == 2 ? B & 1 : 0) * kXTileDoubles;
 #pragma unroll
                         for (int q = 0; q < kRpt; ++q) tl[slot_p * kXPitch + kRpt * rg + q] = combine(acc, q, escale);
                         row_sync(2);
@@ -776,6 +781,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                             }
                             o += (long)(kRole / 16) * n;
                         }
+                        if constexpr (kOutTiles == 1) row_sync(2);   // the tile is free
                     }
                 }
                 // the pencils outside the fixed-point range
@@ -826,9 +832,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaIte
 
 // tensor memory is taken whole: at least 116 KB of shared memory keeps a
 // second CTA off the SM
-template <bool XAX>
+template <bool XAX, int KIND>
 int shared_bytes(int ntype) {
-    const int shm = ntype * kMmaTypeBytes + (XAX ? 4 * kXTileDoubles * (int)sizeof(double) : 0);
+    const int shm = ntype * kMmaTypeBytes + (XAX ? (2 + out_tiles(KIND)) * kXTileDoubles * (int)sizeof(double) : 0);
     return shm < 120 * 1024 ? 120 * 1024 : shm;
 }
 
@@ -852,7 +858,7 @@ long divide(MmaItem &I, int n) {
 
 template <bool XAX, int EPI, int KIND>
 int launch(const MmaItem &I, cudaStream_t st) {
-    const int shm = shared_bytes<XAX>(I.M.ntype);
+    const int shm = shared_bytes<XAX, KIND>(I.M.ntype);
     auto kernel = k_deriv_mma<XAX, EPI, KIND>;
     EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     kernel<<<I.ncta, kMmaThreads, shm, st>>>(I);
@@ -862,7 +868,7 @@ int launch(const MmaItem &I, cudaStream_t st) {
 
 template <bool XAX, int EPI, int KIND>
 int launch(const MmaBatch &b, cudaStream_t st) {
-    const int shm = shared_bytes<XAX>(b.ntype);
+    const int shm = shared_bytes<XAX, KIND>(b.ntype);
     auto kernel = k_batch_deriv_mma<XAX, EPI, KIND>;
     EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     kernel<<<b.ctas, kMmaThreads, shm, st>>>(b.items, b.count);
