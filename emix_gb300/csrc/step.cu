@@ -1155,7 +1155,8 @@ int emix_ctx_launches_per_step(emix_ctx *c) {
     int k = 0;
     const size_t np = c->plan.size();
     for (size_t q = 0; q < np; ++q) {
-        if (fused_with_next(c, q)) ++q;
+        const int fuse = fused_with_next(c, q);
+        if (fuse && !(fuse == 1 && pair_apart(c->plan, q))) ++q;
         ++k;
     }
     return k;
