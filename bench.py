@@ -97,28 +97,28 @@ WALLS = 1
 IMPELLER = True
 
 # FP64 operations (dfma + dadd + dmul thread instructions) per cell a launch
-# covers, measured with ncu on the 192^3 tank (profiles/step_kernels_full_
-# stirred_tank_192.txt, profiles/weno_stage_stirred_tank_192.txt).
+# covers, measured with ncu on the 192^3 tank (profiles/step_tensor_cores_
+# stirred_tank_192.txt; the unfused sgs and flux from their source).  The
+# derivatives run on the tensor cores: theirs is the accumulating add.
 FP64_OPS_PER_CELL = {
-    "weno_stage": 115.4, "grad_x": 18.0, "grad_y": 18.0, "grad_z": 18.0, "grad_yz": 36.1,
-    "div_x": 30.1, "div_y": 30.2, "div_z": 30.2, "flux": 43.0, "sgs": 28.0, "sgs_flux": 58.0,
-    # the RK update: 19.9 in substep 1, 29.5 in substeps 2 and 3 (their um term)
-    "rk_post": 26.3,
+    "weno_stage": 113.0, "grad_x": 0.0, "grad_y": 0.0, "grad_z": 0.0, "grad_yz": 0.0,
+    "div_x": 0.0, "div_y": 5.0, "div_z": 5.0, "flux": 40.0, "sgs": 28.0, "sgs_flux": 55.0,
+    # the RK update: 22.3 in substep 1, 27.5 in substeps 2 and 3 (their um term)
+    "rk_post": 25.8,
 }
 
 # DRAM bytes (read + write) per cell a launch covers, from the same ncu
 # captures; the bench scales them to the 256^3 launch by its cells.
-DRAM_BYTES_PER_CELL = {"weno_stage": 89.1}
+DRAM_BYTES_PER_CELL = {"weno_stage": 88.2}
 
 # where the two tables above come from: ncu captures of the named commands,
 # summarised (command, counters, per-kernel figures) in the profiles files
 CONSTANT_SOURCES = {
-    "fp64_ops_per_cell": "ncu --set full (FP64 fma + add + mul thread instructions per cell), "
+    "fp64_ops_per_cell": "ncu (FP64 fma + add + mul thread instructions per cell), "
                          "python -m emix_gb300.run --n 192 --steps 2 --walls --impeller: "
-                         "profiles/step_kernels_full_stirred_tank_192.txt, "
-                         "profiles/weno_stage_stirred_tank_192.txt",
-    "dram_bytes_per_cell": "ncu --set full (dram__bytes_read.sum + dram__bytes_write.sum per cell of the "
-                           "stage region), same capture: profiles/weno_stage_stirred_tank_192.txt",
+                         "profiles/step_tensor_cores_stirred_tank_192.txt",
+    "dram_bytes_per_cell": "ncu (dram__bytes_read.sum + dram__bytes_write.sum per cell of the "
+                           "stage region), same capture: profiles/step_tensor_cores_stirred_tank_192.txt",
 }
 
 
