@@ -5,7 +5,9 @@
  * Fortran -> C boundary.  Plain pointers and sizes only; no C++ or torch
  * types.  Fields are Fortran column-major (i fastest, index
  * i + nx*(j + ny*k)); multi-component arrays stack components with stride
- * nx*ny*nz.  All arithmetic is IEEE FP64.
+ * nx*ny*nz.  All values are IEEE FP64; derivatives along axes of 40 rows and
+ * more are exact sums of integer digit products on the tensor cores, rounded to
+ * FP64 with the error of an FP64 solve or less.
  *
  * Two families of entry points:
  *   - the reference's own symbols (cudaDeriv, cuDivergence) with byte-identical
