@@ -323,13 +323,9 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                      :: "r"(smem_u32(&s_tmem)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // all columns were asked for, so they begin at 0: a constant, which keeps
     // the tensor-core instructions' operands in uniform registers
     constexpr unsigned tm = 0;
-    if (s_tmem != tm && tid == 0) s_fail = 1;
     const int nblk = M.nblk;
     const int g0 = PER ? -2 : 0;                                   // first and last group of a tile
     const int g1 = PER ? nblk + 2 : (n + 6) / kMmaRows;
@@ -465,8 +461,12 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     if (warp != 2 * kRoleWarps) {
         // the first tile's, by all of them
         scan_tile(cta, 0, warp < 2 * kRoleWarps ? warp : warp - 1, kPencilWarps);
-        asm volatile("bar.sync 3, %0;" :: "n"(32 * kPencilWarps) : "memory");
     }
+    // (the barriers, tensor memory and the operator are on their way meanwhile)
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (s_tmem != tm && tid == 0) s_fail = 1;
 
     if (warp == 2 * kRoleWarps) {
         // ---- the tensor core's warp ----------------------------------------
