@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 
 #include "../../include/emix_gb300.h"
 
@@ -41,6 +42,29 @@ inline int grid_cap(long n, int per_sm, int bs = 256) {
     const long cap = (long)device_sms() * per_sm;
     if (b > cap) b = cap;
     return (int)(b < 1 ? 1 : b);
+}
+
+// A launch that may begin when the blocks of the stream's kernel before it have
+// ended, before that kernel's end is signalled: the launch and the kernel's own
+// setup are out of the way by then.  The kernel calls wait_for_previous() before
+// it reads or writes global memory that others write; it returns once all earlier
+// work is complete and visible.  A 40^3 tank step alone 447 -> 394 us, 97 x 121 x
+// 75 2078 -> 2016, a 64^3 box step 791 -> 750.
+EMIX_DEV void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t shm, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = shm;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // (i, j, k) of cell q of an nx x ny x .. grid of n cells.  In 32 bits where the

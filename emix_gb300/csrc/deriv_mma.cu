@@ -458,6 +458,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         }
     };
     constexpr int kPencilWarps = 2 * kRoleWarps + kScanWarps;   // all but the tensor core's
+    wait_for_previous();   // what is read so far is constant
     if (warp != 2 * kRoleWarps) {
         // the first tile's, by all of them
         scan_tile(cta, 0, warp < 2 * kRoleWarps ? warp : warp - 1, kPencilWarps);
@@ -861,8 +862,7 @@ int launch(const MmaItem &I, cudaStream_t st) {
     const int shm = shared_bytes<XAX, KIND>(I.M.ntype);
     auto kernel = k_deriv_mma<XAX, EPI, KIND>;
     EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
-    kernel<<<I.ncta, kMmaThreads, shm, st>>>(I);
-    EMIX_CUDA_TRY(cudaGetLastError());
+    EMIX_CUDA_TRY(launch_early(kernel, I.ncta, kMmaThreads, (size_t)shm, st, I));
     return EMIX_OK;
 }
 
@@ -871,8 +871,7 @@ int launch(const MmaBatch &b, cudaStream_t st) {
     const int shm = shared_bytes<XAX, KIND>(b.ntype);
     auto kernel = k_batch_deriv_mma<XAX, EPI, KIND>;
     EMIX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
-    kernel<<<b.ctas, kMmaThreads, shm, st>>>(b.items, b.count);
-    EMIX_CUDA_TRY(cudaGetLastError());
+    EMIX_CUDA_TRY(launch_early(kernel, b.ctas, kMmaThreads, (size_t)shm, st, b.items, b.count));
     return EMIX_OK;
 }
 

@@ -5,6 +5,7 @@
 namespace emix {
 
 __global__ void k_imp_clock(ImpClockArgs a) {
+    wait_for_previous();
     imp_clock_tick(a, threadIdx.x);   // one warp
 }
 

@@ -96,6 +96,7 @@ __global__ void k_sgs_setup(const double *__restrict__ xyz, double *__restrict__
 }
 
 __global__ void k_prim(PrimArgs a) {
+    wait_for_previous();
     const long end = a.qend > 0 ? a.qend : a.n;
     for (long q = a.qbeg + blockIdx.x * (long)blockDim.x + threadIdx.x; q < end; q += (long)gridDim.x * blockDim.x)
         prim_cell(a, q);
@@ -103,6 +104,7 @@ __global__ void k_prim(PrimArgs a) {
 __global__ void __launch_bounds__(256, 2) k_flux_all(FluxArgs a) { EMIX_FOR_CELLS(q, a.n) flux_cell(a, q); }
 __global__ void k_sgs_smag(SmagArgs a) { EMIX_FOR_CELLS(q, a.n) smag_cell(a, q); }
 __global__ void __launch_bounds__(256, 2) k_smag_flux(SmagArgs s, FluxArgs f) {
+    wait_for_previous();
     EMIX_FOR_CELLS(q, f.n) smag_flux_cell(s, f, q);
 }
 __global__ void k_sgs_sf(SfArgs a) { EMIX_FOR_CELLS(q, a.n) sf_cell(a, q); }
@@ -114,6 +116,7 @@ __global__ void k_selective(SelArgs a) { EMIX_FOR_CELLS(q, a.n) select_cell(a, q
 // 2.90 (64-bit indices and unscaled sums 3.50, 8 blocks a SM 3.19, one block
 // per 256 cells 3.05).
 __global__ void k_rk_post(RkArgs a) {
+    wait_for_previous();
     const long end = a.qend > 0 ? a.qend : rk_count(a);
     for (long q = a.qbeg + blockIdx.x * (long)blockDim.x + threadIdx.x; q < end; q += (long)gridDim.x * blockDim.x)
         rk_cell(a, q);

@@ -40,10 +40,11 @@ __global__ void k_metric_products(const double *__restrict__ jbn, double *__rest
 int launch_single(const Launch &L, cudaStream_t st) {
     switch (L.kind) {
     case LK_PRIM:
-        k_prim<<<grid_cap(L.prim.n, 64), 256, 0, st>>>(L.prim);
+        EMIX_CUDA_TRY(launch_early(k_prim, grid_cap(L.prim.n, 64), 256, 0, st, L.prim));
         break;
     case LK_PAD:
-        k_ghost_pad<<<cells_grid(L.pad.qend > 0 ? L.pad.qend - L.pad.qbeg : L.pad.ng), 256, 0, st>>>(L.pad);
+        EMIX_CUDA_TRY(launch_early(k_ghost_pad, cells_grid(L.pad.qend > 0 ? L.pad.qend - L.pad.qbeg : L.pad.ng), 256, 0,
+                                   st, L.pad));
         break;
     case LK_WENO:
         return launch_weno_stage(L.weno, st, L.tmap);
@@ -71,13 +72,13 @@ int launch_single(const Launch &L, cudaStream_t st) {
         k_flux_all<<<cells_grid(L.flux.n), 256, 0, st>>>(L.flux);
         break;
     case LK_RK:
-        k_rk_post<<<grid_cap(rk_count(L.rk), 64), 256, 0, st>>>(L.rk);
+        EMIX_CUDA_TRY(launch_early(k_rk_post, grid_cap(rk_count(L.rk), 64), 256, 0, st, L.rk));
         break;
     case LK_BC:
         k_bc<<<cells_grid(bc_count(L.bc)), 256, 0, st>>>(L.bc);
         break;
     case LK_CLOCK:
-        k_imp_clock<<<1, 32, 0, st>>>(L.clock);
+        EMIX_CUDA_TRY(launch_early(k_imp_clock, 1, 32, 0, st, L.clock));
         break;
     case LK_INTERP:
         if (L.interp.phase == 0)
@@ -370,8 +371,7 @@ int launch_fused_pair(const std::vector<Launch> &P, size_t k, cudaStream_t st) {
         return launch_deriv_yz_pair(a.T, b.T, a.nf, b.nf, in, out, a.nx, a.ny, a.nz, st);
     }
     const FluxArgs &fa = P[k + 1].flux;
-    k_smag_flux<<<cells_grid(fa.n), 256, 0, st>>>(L.smag, fa);
-    EMIX_CUDA_TRY(cudaGetLastError());
+    EMIX_CUDA_TRY(launch_early(k_smag_flux, cells_grid(fa.n), 256, 0, st, L.smag, fa));
     return EMIX_OK;
 }
 } // namespace emix
