@@ -71,7 +71,7 @@ EMIX_DEV void prim_adj(const double um[4], double inv_m2, const double lu[3], do
     lum[0] += l0;
 }
 
-// ---- fluxes: lF (15) -> lum(2..5), lu (3), lp, ldvel (9), lvis ---------------
+// ---- fluxes: lF (15) -> lum(2..5) accumulated, lu (3), lp, ldvel (9), lvis ------
 // um = fields 2..5 of the conserved state (rho u, rho v, rho w, T)
 EMIX_DEV void flux_adj(const double um[4], const double u[3], double vs, const double dv[9],
                        double j1, double j5, double j9, double JX, double JY, double JZ,
@@ -80,26 +80,28 @@ EMIX_DEV void flux_adj(const double um[4], const double u[3], double vs, const d
     const double um2 = um[0], um3 = um[1], um4 = um[2], um5 = um[3];
     const double u1 = u[0], u2 = u[1], u3 = u[2];
     const double sxx = j1 * dv[0], syy = j5 * dv[4], szz = j9 * dv[8];
-    const double sxy = j1 * dv[1] + j5 * dv[3];
-    const double sxz = j1 * dv[2] + j9 * dv[6];
-    const double syz = j9 * dv[7] + j5 * dv[5];
+    const double sxy = fma(j1, dv[1], j5 * dv[3]);
+    const double sxz = fma(j1, dv[2], j9 * dv[6]);
+    const double syz = fma(j9, dv[7], j5 * dv[5]);
     const double x0 = lF[0] * JX, y0 = lF[1] * JY, z0 = lF[2] * JZ;
     const double a1 = lF[3] * JX, b1 = lF[4] * JY, c1 = lF[5] * JZ;
     const double a2 = lF[6] * JX, b2 = lF[7] * JY, c2 = lF[8] * JZ;
     const double a3 = lF[9] * JX, b3 = lF[10] * JY, c3 = lF[11] * JZ;
     const double a4 = lF[12] * JX, b4 = lF[13] * JY, c4 = lF[14] * JZ;
-    lum[0] += -x0 - a1 * u1 - a2 * u2 - a3 * u3;
-    lum[1] += -y0 - b1 * u1 - b2 * u2 - b3 * u3;
-    lum[2] += -z0 - c1 * u1 - c2 * u2 - c3 * u3;
-    lum[3] += -(a4 * u1 + b4 * u2 + c4 * u3);
-    lu[0] += -(a1 * um2 + b1 * um3 + c1 * um4) - a4 * um5;
-    lu[1] += -(a2 * um2 + b2 * um3 + c2 * um4) - b4 * um5;
-    lu[2] += -(a3 * um2 + b3 * um3 + c3 * um4) - c4 * um5;
-    lp += -(a1 + b2 + c3);
-    lvs = a1 * 2.0 * sxx + b2 * 2.0 * syy + c3 * 2.0 * szz + (b1 + a2) * sxy + (c1 + a3) * sxz +
-          (c2 + b3) * syz;
-    const double lsxx = 2.0 * vs * a1, lsyy = 2.0 * vs * b2, lszz = 2.0 * vs * c3;
-    const double lsxy = vs * (b1 + a2), lsxz = vs * (c1 + a3), lsyz = vs * (c2 + b3);
+    // lum accumulates, one FMA a term
+    lum[0] = fma(-a1, u1, fma(-a2, u2, fma(-a3, u3, lum[0] - x0)));
+    lum[1] = fma(-b1, u1, fma(-b2, u2, fma(-b3, u3, lum[1] - y0)));
+    lum[2] = fma(-c1, u1, fma(-c2, u2, fma(-c3, u3, lum[2] - z0)));
+    lum[3] = fma(-a4, u1, fma(-b4, u2, fma(-c4, u3, lum[3])));
+    lu[0] = fma(-a1, um2, fma(-b1, um3, fma(-c1, um4, -a4 * um5)));
+    lu[1] = fma(-a2, um2, fma(-b2, um3, fma(-c2, um4, -b4 * um5)));
+    lu[2] = fma(-a3, um2, fma(-b3, um3, fma(-c3, um4, -c4 * um5)));
+    lp = -a1 - b2 - c3;
+    const double txy = b1 + a2, txz = c1 + a3, tyz = c2 + b3;
+    lvs = fma(2.0, fma(a1, sxx, fma(b2, syy, c3 * szz)), fma(txy, sxy, fma(txz, sxz, tyz * syz)));
+    const double vs2 = vs + vs;
+    const double lsxx = vs2 * a1, lsyy = vs2 * b2, lszz = vs2 * c3;
+    const double lsxy = vs * txy, lsxz = vs * txz, lsyz = vs * tyz;
     ldv[0] = j1 * lsxx;
     ldv[4] = j5 * lsyy;
     ldv[8] = j9 * lszz;
@@ -112,29 +114,35 @@ EMIX_DEV void flux_adj(const double um[4], const double u[3], double vs, const d
 }
 
 // ---- Smagorinsky: lvis -> ldvel (+=), returns d vis / d Cs * lvis ----------
+// vis = c4 + (Cs Delta)^2 root, root^2 = 2 (sxx^2 + syy^2 + szz^2) + sxy^2 + sxz^2 +
+// syz^2: d root = (2 sxx dsxx + ... + sxy dsxy + ...) / root.  With the strain
+// pieces of the forward kernel and 1/root by its own step, 45 FP64 operations
+// (77 with root and its reciprocal, halved shears and sums started from zero).
 EMIX_DEV double smag_adj(const double dv[9], double j1, double j5, double j9, double cs,
                          double delta, double lvis, double ldv[9]) {
-    const double ux = j1 * dv[0], vx = j1 * dv[1], wx = j1 * dv[2];
-    const double uy = j5 * dv[3], vy = j5 * dv[4], wy = j5 * dv[5];
-    const double uz = j9 * dv[6], vz = j9 * dv[7], wz = j9 * dv[8];
-    const double s12 = 0.5 * (uy + vx), s13 = 0.5 * (uz + wx), s23 = 0.5 * (vz + wy);
-    const double ss = ux * ux + vy * vy + wz * wz + 2.0 * (s12 * s12 + s13 * s13 + s23 * s23);
-    const double root = sqrt_fast(2.0 * ss);
-    const double cd = cs * delta;
-    if (root > 0.0) {
-        const double lss = lvis * cd * cd * rcp_fast(root);
-        const double l12 = 2.0 * lss * s12, l13 = 2.0 * lss * s13, l23 = 2.0 * lss * s23;
-        ldv[0] += j1 * 2.0 * ux * lss;
-        ldv[4] += j5 * 2.0 * vy * lss;
-        ldv[8] += j9 * 2.0 * wz * lss;
-        ldv[3] += j5 * l12;   // uy
-        ldv[1] += j1 * l12;   // vx
-        ldv[6] += j9 * l13;   // uz
-        ldv[2] += j1 * l13;   // wx
-        ldv[7] += j9 * l23;   // vz
-        ldv[5] += j5 * l23;   // wy
-    }
-    return lvis * 2.0 * cs * delta * delta * root;
+    const double sxx = j1 * dv[0], syy = j5 * dv[4], szz = j9 * dv[8];
+    const double sxy = fma(j1, dv[1], j5 * dv[3]);
+    const double sxz = fma(j1, dv[2], j9 * dv[6]);
+    const double syz = fma(j9, dv[7], j5 * dv[5]);
+    const double nn = fma(szz, szz, fma(syy, syy, sxx * sxx));
+    const double x = fma(2.0, nn, fma(syz, syz, fma(sxz, sxz, sxy * sxy)));
+    const double m = lvis * delta * delta;
+    // x > 0 by its bits (NaN: not)
+    if ((unsigned long long)__double_as_longlong(x) - 1 >= 0x7ff0000000000000ull) return m * (2.0 * cs) * x;
+    const double ri = rsqrt_fast(x);
+    const double g = m * (cs * cs) * ri, g2 = g + g;
+    const double gx = g2 * sxx, gy = g2 * syy, gz = g2 * szz;
+    const double gxy = g * sxy, gxz = g * sxz, gyz = g * syz;
+    ldv[0] = fma(j1, gx, ldv[0]);
+    ldv[4] = fma(j5, gy, ldv[4]);
+    ldv[8] = fma(j9, gz, ldv[8]);
+    ldv[3] = fma(j5, gxy, ldv[3]);   // uy
+    ldv[1] = fma(j1, gxy, ldv[1]);   // vx
+    ldv[6] = fma(j9, gxz, ldv[6]);   // uz
+    ldv[2] = fma(j1, gxz, ldv[2]);   // wx
+    ldv[7] = fma(j9, gyz, ldv[7]);   // vz
+    ldv[5] = fma(j5, gyz, ldv[5]);   // wy
+    return m * (2.0 * cs) * (x * ri);
 }
 
 // ---- RK conversions and impeller -------------------------------------------
@@ -160,13 +168,16 @@ EMIX_DEV void convert_adj(const RkArgs &a, long q, const double v_in[5], const d
     }
     // conversions at v
     const double r = v[0], rr = rcp_fast(r), mk = a.mask[q];
-    double lr = lo[0] + lp * a.inv_m2;
+    double lr = fma(lp, a.inv_m2, lo[0]);
     for (int d = 0; d < 3; ++d) {
+        // inside the clip the velocity's adjoint passes; outside (by the bits;
+        // NaN too) the momentum is the bound times the density
         const double c = v[d + 1] * rr;
-        const double gd = (c > -6.0 && c < 6.0) ? 1.0 : 0.0;
-        const double cl = fmax(-6.0, fmin(6.0, c));
-        lr += lo[d + 1] * mk * (cl - gd * c) - lu[d] * gd * mk * c * rr;
-        lv[d + 1] = lo[d + 1] * gd * mk + lu[d] * gd * mk * rr;
+        const bool in = (__double_as_longlong(c) & 0x7fffffffffffffffLL) < 0x4018000000000000LL;   // |c| < 6
+        const double g = in ? mk : 0.0, w = lu[d] * rr;
+        lv[d + 1] = g * (lo[d + 1] + w);
+        lr = fma(-(g * w), c, lr);
+        if (!in) lr = fma(lo[d + 1] * mk, fmax(-6.0, fmin(6.0, c)), lr);
     }
     lv[4] = lo[4];
     lv[0] = lr;

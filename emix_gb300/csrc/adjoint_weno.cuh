@@ -31,9 +31,11 @@ __global__ void __launch_bounds__(256) k_adj_weno(WenoAdjArgs A) {
     const long ng = (long)nxg * nyg * nzg, nv = (long)nx * ny * nz;
     const long cnt = (long)A.rn[0] * A.rn[1] * A.rn[2];
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < cnt; t += (long)gridDim.x * blockDim.x) {
-        const int X = A.r0[0] + (int)(t % A.rn[0]);
-        const int Y = A.r0[1] + (int)((t / A.rn[0]) % A.rn[1]);
-        const int Z = A.r0[2] + (int)(t / ((long)A.rn[0] * A.rn[1]));
+        int X, Y, Z;
+        cell_of(t, cnt, A.rn[0], A.rn[1], X, Y, Z);
+        X += A.r0[0];
+        Y += A.r0[1];
+        Z += A.r0[2];
         const long id = X + (long)nxg * (Y + (long)nyg * Z);
         double lo;
         if (A.stage == 3) {
@@ -55,8 +57,12 @@ __global__ void __launch_bounds__(256) k_adj_weno(WenoAdjArgs A) {
             A.lphiin[id] += 0.25 * lo;
             lrs = -0.25 * A.dt * lo;
         } else {
-            A.lphi0[id] += lo / 3.0;
-            A.lphiin[id] += 2.0 * lo / 3.0;
+            // lo / 3: the product with 1/3 and its remainder (a division is 8
+            // operations on the FP64 pipe, which bounds this)
+            double th = lo * (1.0 / 3.0);
+            th = fma(fma(-3.0, th, lo), 1.0 / 3.0, th);
+            A.lphi0[id] += th;
+            A.lphiin[id] += th + th;
             lrs = -(2.0 / 3.0) * A.dt * lo;
         }
         const long iv = mirror(X, g, nx) + (long)nx * (mirror(Y, g, ny) + (long)ny * mirror(Z, g, nz));
@@ -88,7 +94,8 @@ __global__ void k_adj_weno_dphi(const double *lD, double *lphi, int nxg, int nyg
     const int L3[3] = {nxg, nyg, nzg};
     const long s3[3] = {1, nxg, (long)nxg * nyg};
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < ng; q += (long)gridDim.x * blockDim.x) {
-        const int c3[3] = {(int)(q % nxg), (int)((q / nxg) % nyg), (int)(q / ((long)nxg * nyg))};
+        int c3[3];
+        cell_of(q, ng, nxg, nyg, c3[0], c3[1], c3[2]);
         double acc = 0.0;
         for (int d = 0; d < 3; ++d) {
             const double *D = lD + d * ng;
@@ -108,7 +115,8 @@ __global__ void k_adj_unpad(const double *lpad, double *lint, int g, int nx, int
     const long n = (long)nx * ny * nz;
     const int nxg = nx + 2 * g, nyg = ny + 2 * g;
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-        const int c3[3] = {(int)(q % nx), (int)((q / nx) % ny), (int)(q / ((long)nx * ny))};
+        int c3[3];
+        cell_of(q, n, nx, ny, c3[0], c3[1], c3[2]);
         const int n3[3] = {nx, ny, nz};
         int img[3][3], cnt[3];
         for (int d = 0; d < 3; ++d) {
@@ -168,7 +176,8 @@ __global__ void __launch_bounds__(256) k_objective(ObjArgs A) {
         // interface area
         const double ph = A.phi[q];
         if (fabs(ph) >= A.eps) continue;
-        const int c3[3] = {(int)(q % nx), (int)((q / nx) % ny), (int)(q / ((long)nx * ny))};
+        int c3[3];
+        cell_of(q, n, nx, ny, c3[0], c3[1], c3[2]);
         const int n3[3] = {nx, ny, nz};
         const long s3[3] = {1, nx, (long)nx * ny};
         const double jd[3] = {A.jbn[q], A.jbn[4 * n + q], A.jbn[8 * n + q]};
