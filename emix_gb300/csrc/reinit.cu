@@ -277,7 +277,7 @@ int reinit_impl(double *phi, const double *jbn, const double *dmins, double dX, 
     a.dt = 0.5 * deltamin; a.ref_bugs = ref_bugs;
     const int gx = (nxg + kMX - 1) / kMX, gy = (nyg + kMY - 1) / kMY;
     if (gy > 65535) return EMIX_ERR_ARG;
-    const int gz = march_chunks((long)gx * gy, nzg);
+    const int gz = march_chunks((long)gx * gy, nzg, 3);
     const dim3 grid(gx, gy, gz);
     k_reinit_scales<<<grid_r(ng), 256, 0, st>>>(jbn, reinterpret_cast<double2 *>(scr), 1.0 / dX, 1.0 / dY, 1.0 / dZ, ng);
     for (int it = 0; it < iters; ++it) {

@@ -60,7 +60,7 @@ bool weno_tma_map(CUtensorMap *m, const WenoArgs &a) {
 int launch_weno_march(const WenoArgs &a, cudaStream_t st, const CUtensorMap *tmap) {
     const int gx = (a.rn[0] + kMX - 1) / kMX, gy = (a.rn[1] + kMY - 1) / kMY;
     if (gy > 65535) return EMIX_ERR_ARG;
-    const dim3 grid(gx, gy, (unsigned)march_chunks((long)gx * gy, a.rn[2]));
+    const dim3 grid(gx, gy, (unsigned)march_chunks((long)gx * gy, a.rn[2], 4));
     if (tmap) k_weno_march_tma<<<grid, kNT, 0, st>>>(*tmap, a);
     else k_weno_march<<<grid, kNT, 0, st>>>(a);
     EMIX_CUDA_TRY(cudaGetLastError());

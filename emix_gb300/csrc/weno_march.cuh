@@ -110,19 +110,23 @@ EMIX_DEV void weno_z_general(const double *phi, long id, int Z, int nzg, bool le
     }
 }
 
-// z chunks of a marching launch over `cols` columns of nz planes.  Short
-// chunks pay their start (the window of differences, the first copies: a tenth
-// of a plane) more often, long ones leave SMs idle behind the most loaded one
-// (a quarter of a chunk on average: blocks land unevenly, and a lone block is
-// no faster per plane than four).  With P planes per SM the sum of both,
-// 0.1 P / c + c / 4, is least at c = sqrt(P / 2.5).  Lengths of 1 to 64 planes
-// measured: 40^3 1 (0.138 ms a step, 12 planes 0.355), 64^3 1-2 (0.318), 96^3
-// 4 (0.822, this rule 0.831, one block per SM 1.05), 128^3 5 (1.710), 160 x 160
-// x 128 6 (2.569); the reinitialisation's stages alike (96^3 3, 130 x 118 x 106
-// 5).
-inline int march_chunks(long cols, int nz) {
-    const double planes = (double)cols * nz / device_sms();
+// z chunks of a marching launch over `cols` columns of nz planes, `per_sm` blocks
+// of which an SM holds.  Short chunks pay their start (the window of differences,
+// the first copies: a tenth of a plane) more often, long ones leave SMs idle
+// behind the most loaded one (a quarter of a chunk on average: blocks land
+// unevenly).  With P planes per SM the sum of both, 0.1 P / c + c / 4, is least at
+// c = sqrt(P / 2.5); below P = 10 one plane measured best.  Lengths of 1 to 64
+// planes, ms: 40^3 1 (0.138 a step, 12 planes 0.355), 64^3 1-2 (0.318), 96^3 4
+// (0.822, 3 0.831, one block per SM 1.05), 128^3 5 (1.710), 160 x 160 x 128 6
+// (2.569); reinitialisation 70 x 81 x 32 1 (3.52, 2 planes 4.56), 106^3 3, 140 x 128
+// x 116 5.  Blocks of one plane that are a few more than are resident run a second
+// time for those few: two planes where that makes two blocks an SM
+// (reinitialisation 37 x 50 x 42: 2.78 -> 2.48).
+inline int march_chunks(long cols, int nz, int per_sm) {
+    const long sms = device_sms();
+    const double planes = (double)cols * nz / sms;
     int c = (int)(sqrt(planes / 2.5) + 0.5);
+    if (planes < 10.0) c = cols * nz > 1.07 * per_sm * sms && cols * ((nz + 1) / 2) <= 2 * sms ? 2 : 1;
     if (c < nz / 65535 + 1) c = nz / 65535 + 1;
     return (nz + c - 1) / c;
 }
