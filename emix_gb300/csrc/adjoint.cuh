@@ -19,12 +19,10 @@
 namespace emix {
 
 // out = D^T in (acc = 0) or out += D^T in (acc = 1) along `axis`, for nf <= 6
-// fields; w is scratch of the size of in.  Closed tables of kMmaMinN rows and
-// more run on the tensor cores (`sweeps`: not); otherwise, with maps (y or z, a
-// closed table) the rows come by TMA through them, the same values bit for bit
-// as without.
+// fields; w is scratch of the size of in.  With maps (y or z, a closed
+// table) the rows come by TMA through them, the same values bit for bit.
 int launch_deriv_t(const DerivTTable &T, int axis, int acc, int nf, const double *const *in,
                    double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st,
-                   const PencilMaps *maps = nullptr, bool sweeps = false);
+                   const PencilMaps *maps = nullptr);
 
 } // namespace emix

@@ -9,10 +9,8 @@
 // antisymmetric 5-point stencil).  The cyclic scheme is anti-self-adjoint (D^T = -D) and uses the
 // forward kernels with a negated table.  Given tensor maps, the y and z
 // passes run k_deriv_t_yz_tma (deriv_tma.cu), the same arithmetic on rows
-// staged by TMA.  Pencils of kMmaMinN rows and more go to the tensor cores in
-// the reverse sweep (deriv_mma.cu).
+// staged by TMA.
 #include "adjoint.cuh"
-#include "deriv_mma.cuh"
 
 namespace emix {
 
@@ -38,7 +36,66 @@ __global__ void __launch_bounds__(128) k_deriv_t(DerivTTable T, PencilFields F, 
     const double *in = pick(F.in, f) + base;
     double *w = pick(F.w, f) + base;
     double *out = pick(F.out, f) + base;
-    deriv_t_pencil<ACC>(T, in, w, out, s);
+    const DerivTRow *R = T.rows;
+    const double *BT = T.bt;
+    // forward: y_i = r_i ib_i - m_i y_{i-1}
+    double y = 0.0;
+    for (int i = 0; i < L; ++i) {
+        const DerivTRow r = R[i];
+        y = fma(-r.m, y, in[i * s] * r.ib);
+        w[i * s] = y;
+    }
+    // backward: z_i = y_i - g_i z_{i+1}; zq[t] = z_{i+t}; out_j, j = i + 3,
+    // once z_i is known.  Three branch-free runs of j: the closure rows at the
+    // top, the interior rows (4 operations on the antisymmetric stencil), the
+    // closure rows at the bottom.
+    double zq[7];
+#pragma unroll
+    for (int t = 0; t < 7; ++t) zq[t] = 0.0;
+    double z = 0.0;
+    auto advance = [&](int i) {
+#pragma unroll
+        for (int t = 6; t > 0; --t) zq[t] = zq[t - 1];
+        if (i >= 0) {
+            const double wi = w[i * s];
+            z = (i == L - 1) ? wi : fma(-R[i].g, z, wi);
+            zq[0] = z;
+        } else {
+            zq[0] = 0.0;
+        }
+    };
+    auto put = [&](int j, double o) {
+        if (ACC) out[j * s] += o;
+        else out[j * s] = o;
+    };
+    auto general = [&](int j) {
+        const double *b = BT + 7 * (long)j;
+        double o = b[0] * zq[0];
+#pragma unroll
+        for (int t = 1; t < 7; ++t) o = fma(b[t], zq[t], o);
+        put(j, o);
+    };
+    const bool fast = T.jlo <= T.jhi;
+    const int jtop = fast ? T.jhi : -1;   // rows above jtop: closure rows
+    const int jbot = fast ? T.jlo : 0;    // rows below jbot: closure rows
+    int i = L - 1;
+    for (; i >= -3 && i + 3 > jtop; --i) {
+        advance(i);
+        if (i + 3 < L) general(i + 3);
+    }
+    if (fast) {
+        for (; i + 3 >= jbot; --i) {
+            advance(i);
+            // accumulated: the add folds into the stencil's second FMA
+            const long js = (long)(i + 3) * s;
+            if (ACC) out[js] = fma(T.ta, zq[2] - zq[4], fma(T.tb, zq[1] - zq[5], out[js]));
+            else out[js] = fma(T.ta, zq[2] - zq[4], T.tb * (zq[1] - zq[5]));
+        }
+    }
+    for (; i >= -3; --i) {
+        advance(i);
+        general(i + 3);
+    }
 }
 
 // x pencils (contiguous rows): a warp owns 32 pencils and stages 32-row
@@ -171,9 +228,8 @@ __global__ void __launch_bounds__(128) k_deriv_t_x(DerivTTable T, PencilFields F
 
 int launch_deriv_t(const DerivTTable &T, int axis, int acc, int nf, const double *const *in,
                    double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st,
-                   const PencilMaps *maps, bool sweeps) {
+                   const PencilMaps *maps) {
     if (nf < 1 || nf > kMaxFields || axis < 0 || axis > 2) return EMIX_ERR_ARG;
-    if (T.mma && !sweeps) return launch_deriv_t_mma(T, axis, acc, nf, in, w, out, nx, ny, nz, st);
     if (maps && axis != 0 && !T.periodic)
         return launch_deriv_t_yz_tma(T, *maps, acc, nf, in, w, out, nx, ny, nz, st);
     if (T.periodic) {
@@ -238,10 +294,8 @@ int deriv_t_dev(int scheme, int axis, int nf, double *out, const double *in, dou
     }
     PencilMaps M;
     if (tma && !pencil_tma_maps(&M, axes, nf, ins, ws, outs, nx, ny, nz)) return EMIX_ERR_ARG;
-    // along y and z the sweeps at every length: the form with rows by TMA gives
-    // their bits
     return launch_deriv_t(T, axis, accumulate, nf, ins, ws, outs, nx, ny, nz, (cudaStream_t)stream,
-                          tma ? &M : nullptr, axis != 0);
+                          tma ? &M : nullptr);
 }
 
 } // namespace

@@ -258,7 +258,6 @@ struct DerivTTable {
     int jlo, jhi;
     double ta, tb;
     DerivTable neg;
-    const struct MmaTable *mma;   // on the tensor cores (closed, kMmaMinN rows and more), or null
 };
 int get_deriv_t_table(int scheme, int n, double h, DerivTTable *out);
 

@@ -500,71 +500,4 @@ int launch_deriv_yz_pair(const DerivTable &Ty, const DerivTable &Tz, int nfa, in
                          const double *const *in, double *const *out, int nx, int ny, int nz,
                          cudaStream_t st);
 
-// D^T of one pencil (rows `s` apart) by one thread: forward sweep of A^T into
-// the scratch w, backward sweep with a 7-value register window
-template <int ACC>
-EMIX_DEV void deriv_t_pencil(const DerivTTable &T, const double *in, double *w, double *out, long s) {
-    const int n = T.n;
-    const DerivTRow *R = T.rows;
-    const double *BT = T.bt;
-    // forward: y_i = r_i ib_i - m_i y_{i-1}
-    double y = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const DerivTRow r = R[i];
-        y = fma(-r.m, y, in[i * s] * r.ib);
-        w[i * s] = y;
-    }
-    // backward: z_i = y_i - g_i z_{i+1}; zq[t] = z_{i+t}; out_j, j = i + 3,
-    // once z_i is known.  Three branch-free runs of j: the closure rows at the
-    // top, the interior rows (4 operations on the antisymmetric stencil), the
-    // closure rows at the bottom.
-    double zq[7];
-#pragma unroll
-    for (int t = 0; t < 7; ++t) zq[t] = 0.0;
-    double z = 0.0;
-    auto advance = [&](int i) {
-#pragma unroll
-        for (int t = 6; t > 0; --t) zq[t] = zq[t - 1];
-        if (i >= 0) {
-            const double wi = w[i * s];
-            z = (i == n - 1) ? wi : fma(-R[i].g, z, wi);
-            zq[0] = z;
-        } else {
-            zq[0] = 0.0;
-        }
-    };
-    auto put = [&](int j, double o) {
-        if (ACC) out[j * s] += o;
-        else out[j * s] = o;
-    };
-    auto general = [&](int j) {
-        const double *b = BT + 7 * (long)j;
-        double o = b[0] * zq[0];
-#pragma unroll
-        for (int t = 1; t < 7; ++t) o = fma(b[t], zq[t], o);
-        put(j, o);
-    };
-    const bool fast = T.jlo <= T.jhi;
-    const int jtop = fast ? T.jhi : -1;   // rows above jtop: closure rows
-    const int jbot = fast ? T.jlo : 0;    // rows below jbot: closure rows
-    int i = n - 1;
-    for (; i >= -3 && i + 3 > jtop; --i) {
-        advance(i);
-        if (i + 3 < n) general(i + 3);
-    }
-    if (fast) {
-        for (; i + 3 >= jbot; --i) {
-            advance(i);
-            // accumulated: the add folds into the stencil's second FMA
-            const long js = (long)(i + 3) * s;
-            if (ACC) out[js] = fma(T.ta, zq[2] - zq[4], fma(T.tb, zq[1] - zq[5], out[js]));
-            else out[js] = fma(T.ta, zq[2] - zq[4], T.tb * (zq[1] - zq[5]));
-        }
-    }
-    for (; i >= -3; --i) {
-        advance(i);
-        general(i + 3);
-    }
-}
-
 } // namespace emix

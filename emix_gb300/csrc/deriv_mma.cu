@@ -43,12 +43,6 @@
 // 2-norm: A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 ->
 // 9.4e-16, C 5.7e-15 -> 3.4e-15.
 //
-// D^T of the closed schemes (the adjoint) is a table of the same form and one
-// FP64 operation more on the ends' rows: the gradient of a 96^3 tank objective
-// over three steps 18.7 -> 16.9 ms; error against a dense transpose no larger
-// than the sweeps' (192 rows: A 8.0e-16 -> 5.4e-16, B 4.0e-16 -> 3.2e-16, C
-// 8.4e-16 -> 6.2e-16).
-//
 // Pencils with infinities or NaN, or of magnitudes whose fixed-point
 // exponents would leave the FP64 range, take the scalar sweep (deriv.cuh)
 // after the tile.
@@ -82,19 +76,19 @@ constexpr int kAccCols = kMmaDig * kMmaRows;
 constexpr int kHighRing = 7, kLowRing = 6;
 constexpr int kHighCol = 2 * kAccCols, kLowCol = kHighCol + kHighRing * 24;
 constexpr int kTmemCols = 512;
-// Kinds of pencils: closed, closed under D^T, cyclic, and short cyclic ones of whole groups, all of
+// Kinds of pencils: closed, cyclic, and short cyclic ones of whole groups, all of
 // whose groups are held in tensor memory at once and read round the cycle by the
 // blocks, instead of five of them converted twice.  At least three groups (which
 // wrap once) and at most four (which leave two places for the next tile's).  5
 // fields of 64^3, us: x 28.2 -> 22.6, y and z 25.1 -> 20.7.  A kind of its own:
 // tested at run time it costs the other cyclic pencils 2% (256^3 562 -> 574).
-constexpr int kClosed = 0, kCyclic = 1, kRound = 2, kTransposed = 3;
+constexpr int kClosed = 0, kCyclic = 1, kRound = 2;
 constexpr int kMmaRoundN = 64;
 static_assert(kMmaMinN > 2 * kMmaRows && kMmaRoundN / kMmaRows < kLowRing, "kMmaRoundN");
 // x: tiles of finished blocks.  A closed table's seven block types leave 28 KB of
 // L1 beside two of them, 60 KB beside one, and what is in flight lives there: 5
 // fields of 256^3 0.610 ms with two, 0.537 with one and another barrier a block.
-constexpr int out_tiles(int kind) { return kind == kClosed || kind == kTransposed ? 1 : 2; }
+constexpr int out_tiles(int kind) { return kind == kClosed ? 1 : 2; }
 int kind_of(int n, bool periodic) {
     return !periodic ? kClosed : (n % kMmaRows == 0 && n <= kMmaRoundN ? kRound : kCyclic);
 }
@@ -736,17 +730,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                     if constexpr (!XAX) {
                         if (cur.live && !sc.scalar && ok) {
                             double *o = cur.out + (long)row * s;
-                            if (KIND == kTransposed && (b < M.nlow || b >= nblk - M.nhigh)) {
-                                // the ends' blocks: the row sums' share
-#pragma unroll
-                                for (int q = 0; q < kRpt; ++q) {
-                                    if (row + q >= n) break;
-                                    const long at = (long)(row + q) * s;
-                                    double r = fma(M.sigma[row + q], cur.in[at], combine(acc, q, escale));
-                                    if constexpr (EPI == EPI_ACCUM) r += old[q];
-                                    cur.out[at] = r;
-                                }
-                            } else if (row + kRpt <= n) {
+                            if (row + kRpt <= n) {
 #pragma unroll
                                 for (int q = 0; q < kRpt; ++q) {
                                     double r = combine(acc, q, escale);
@@ -775,8 +759,6 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                             const int pp = (rtid >> 4) + (kRole / 16) * q;
                             if (frow < n && cur.p0 + pp < np && !s_scalar[pp] && ok) {
                                 double r = tl[pp * kXPitch + (rtid & 15)];
-                                if (KIND == kTransposed && (b < M.nlow || b >= nblk - M.nhigh))
-                                    r = fma(M.sigma[frow], cur.in[(long)(cur.p0 + pp) * n + frow], r);
                                 if (EPI == EPI_ACCUM) r += *o;
                                 *o = r;
                             }
@@ -789,10 +771,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                 if (rg == 0 && sc.scalar && cur.live && ok && cur.b0 == 0) {
                     const long x = XAX ? cur.wofs : 0;
                     double *w = pick(F.w, cur.field) + cur.wofs;
-                    if constexpr (KIND == kTransposed)
-                        deriv_t_pencil<EPI == EPI_ACCUM>(I.TT, cur.in + x, w, cur.out + x, s);
-                    else
-                        deriv_pencil<EPI>(I.T, cur.in + x, w, cur.out + x, s);
+                    deriv_pencil<EPI>(I.T, cur.in + x, w, cur.out + x, s);
                 }
                 if constexpr (XAX) row_sync(2);   // s_scalar is free
             }
@@ -878,10 +857,8 @@ int launch(const MmaBatch &b, cudaStream_t st) {
 // the variant for an item or a batch of items
 template <bool XAX, int EPI, class W>
 int launch_kind(int kind, const W &w, cudaStream_t st) {
-    if constexpr (std::is_same<W, MmaItem>::value) {   // (a batch holds pencils of all lengths, of D)
+    if constexpr (std::is_same<W, MmaItem>::value)   // (a batch holds pencils of all lengths)
         if (kind == kRound) return launch<XAX, EPI, kRound>(w, st);
-        if (kind == kTransposed) return launch<XAX, EPI, kTransposed>(w, st);
-    }
     return kind == kCyclic ? launch<XAX, EPI, kCyclic>(w, st) : launch<XAX, EPI, kClosed>(w, st);
 }
 
@@ -946,14 +923,6 @@ int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, 
     MmaItem I = mma_item(T, M, axis, fields_of(nf, in, w, out), nf, nx, ny, nz);
     divide(I, device_sms());
     return launch_variant(axis == 0, epi, kind_of(T.n, M.periodic != 0), I, st);
-}
-
-int launch_deriv_t_mma(const DerivTTable &T, int axis, int acc, int nf, const double *const *in, double *const *w,
-                       double *const *out, int nx, int ny, int nz, cudaStream_t st) {
-    MmaItem I = mma_item(DerivTable{}, *T.mma, axis, fields_of(nf, in, w, out), nf, nx, ny, nz);
-    I.TT = T;
-    divide(I, device_sms());
-    return launch_variant(axis == 0, acc ? EPI_ACCUM : EPI_STORE, kTransposed, I, st);
 }
 
 int deriv_mma_timeouts(int *count) {

@@ -45,16 +45,12 @@ struct MmaTable {
     int nlow, nhigh;      // blocks of their own type at the ends; type nlow is the interior's
     int se;               // scale exponent of the entries
     const unsigned short *b;   // ntype x kMmaTypeBytes, f16
-    const double *sigma;       // D^T: the row sums, n (zero but in the ends' blocks)
 };
 
-// The transpose of a closed operator takes the same form less its row sums
-// sigma_j (zero away from the ends): (D^T f)_j = sum_k E'_{jk} d_k + sigma_j f_j.
-//
-// Tensor-core table of (scheme, n, sign h) or of its transpose (kept for the
-// life of the process); null below kMmaMinN rows and where the operator does not fit the
+// Tensor-core table of (scheme, n, sign h) (kept for the life of the
+// process); null below kMmaMinN rows and where the operator does not fit the
 // form above (the callers then keep the sweeps).
-int get_mma_table(int scheme, int n, double h, double sign, bool transposed, const MmaTable **out);
+int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out);
 
 // Whether a derivative goes to the tensor cores: by the length of its
 // pencils.  Measured against the sweeps (us a launch, 3 or 5 fields, closed /
@@ -70,14 +66,9 @@ inline bool deriv_on_mma(const DerivTable &T) { return T.mma != nullptr; }
 int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
                      double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st);
 
-// launch_deriv_t on the tensor cores (T.mma not null)
-int launch_deriv_t_mma(const DerivTTable &T, int axis, int acc, int nf, const double *const *in, double *const *w,
-                       double *const *out, int nx, int ny, int nz, cudaStream_t st);
-
 // One derivative of nf fields of a grid, and the CTAs that walk its tiles.
 struct MmaItem {
     DerivTable T;
-    DerivTTable TT;           // D^T
     MmaTable M;
     PencilFields F;
     int np, ntile, nf, nx;    // pencils, tiles of them, fields

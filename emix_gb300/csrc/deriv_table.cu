@@ -212,7 +212,7 @@ std::map<TableKey, DerivTable> g_tables;   // device buffers live until process 
 } // namespace
 
 int get_table_signed(int scheme, int n, double h, double sign, DerivTable *out);
-int get_mma_table(int scheme, int n, double h, double sign, bool transposed, const MmaTable **out);
+int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out);
 
 int get_deriv_table(int scheme, int n, double h, DerivTable *out) {
     if (!(h > 0.0)) return EMIX_ERR_ARG;
@@ -278,7 +278,7 @@ int get_table_signed(int scheme, int n, double h, double sign, DerivTable *out) 
     t.zz = t.u0 + n;
     t.urows = reinterpret_cast<const DerivRowU *>(t.zz + n);
     t.u0s = t.zz + 5 * (size_t)n;
-    rc = get_mma_table(scheme, n, h, sign, false, &t.mma);
+    rc = get_mma_table(scheme, n, h, sign, &t.mma);
     if (rc) return rc;
     g_tables[key] = t;
     *out = t;
@@ -531,7 +531,6 @@ int get_deriv_t_table(int scheme, int n, double h, DerivTTable *out) {
         EMIX_CUDA_TRY(cudaMemcpy(buf, host.data(), nd * sizeof(double), cudaMemcpyHostToDevice));
         t.rows = reinterpret_cast<const DerivTRow *>(buf);
         t.bt = buf + 3 * (size_t)n;
-        if ((rc = get_mma_table(scheme, n, h, 1.0, true, &t.mma))) return rc;
         // the run of rows around the middle equal to the middle row, when
         // that row is the antisymmetric 5-point stencil
         const double *mid = bt.data() + 7 * (size_t)(n / 2);
@@ -613,48 +612,25 @@ public:
             bet_[j] = 1 - R_[j - 1].c * gam_[j];
         }
     }
-    // D_{im} for m in [m0, m0 + d.size()), the others vanish
-    void values(int i, int &m0, std::vector<real> &d) const {
+    // E_{ik} for k in [k0, k0 + cnt); entries beyond reach are added to the ends
+    void row(int i, int k0, int cnt, std::vector<real> &e) const {
+        constexpr int W = 48;   // 0.38^48 = 2^-67
         const int lo = std::max(0, i - W), hi = std::min(n_ - 1, i + W);
         std::vector<real> y(hi - lo + 1, real(0));
         real w = 1 / bet_[i];
         y[i - lo] = w;
         for (int j = i + 1; j <= hi; ++j) y[j - lo] = w = -R_[j - 1].c * w / bet_[j];
         for (int j = hi - 1; j >= lo; --j) y[j - lo] -= gam_[j + 1] * y[j + 1 - lo];
-        m0 = lo - 8;
-        const int m1 = hi + 8;
-        d.assign(m1 - m0 + 1, real(0));
+        const int m0 = lo - 8, m1 = hi + 8;
+        std::vector<real> d(m1 - m0 + 1, real(0));
         for (int j = lo; j <= hi; ++j)
             for (int k = 0; k < 7; ++k) {
                 const int m = R_[j].first + k;
                 if (m >= m0 && m <= m1) d[m - m0] += y[j - lo] * R_[j].q[k];
             }
-    }
-    // the same of the transpose, less its row sums, which are returned
-    real values_t(int j, int &m0, std::vector<real> &d) const {
-        const int lo = std::max(0, j - W), hi = std::min(n_ - 1, j + W);
-        m0 = lo;
-        d.assign(hi - lo + 1, real(0));
-        real sum = 0;
-        for (int i = lo; i <= hi; ++i) {
-            std::vector<real> &v = rows_[i];   // formed once: many columns meet it
-            int v0 = std::max(0, i - W) - 8;
-            if (v.empty()) values(i, v0, v);
-            if (j >= v0 && j < v0 + (int)v.size()) sum += d[i - lo] = v[j - v0];
-        }
-        return sum;
-    }
-    // E_{ik} for k in [k0, k0 + cnt) of D (t: of its transpose less the row sums,
-    // returned); entries beyond reach are added to the ends
-    real row(int i, int k0, int cnt, std::vector<real> &e, bool t) const {
-        std::vector<real> d;
-        int m0;
-        real sigma = 0;
-        if (t) sigma = values_t(i, m0, d);
-        else values(i, m0, d);
         e.assign(cnt, real(0));
         real s = 0;   // from the right: sum of D_{im}, m > k, for k >= i
-        for (int m = m0 + (int)d.size() - 1; m > i; --m) {
+        for (int m = m1; m > i; --m) {
             s += d[m - m0];
             e[std::min(std::max(m - 1 - k0, 0), cnt - 1)] += s;
         }
@@ -663,15 +639,12 @@ public:
             s += d[m - m0];
             e[std::min(std::max(m - k0, 0), cnt - 1)] -= s;
         }
-        return sigma;
     }
 
 private:
-    static constexpr int W = 48;   // 0.38^48 = 2^-67
     int n_;
     std::vector<ExactRow> R_;
     std::vector<real> bet_, gam_;
-    mutable std::map<int, std::vector<real>> rows_;
 };
 
 // an integer of at most 11 bits as f16
@@ -690,17 +663,16 @@ unsigned short half_bits(int v) {
 constexpr int kMmaEnd = 44;
 
 struct MKey {
-    int dev, scheme, n, transposed;
+    int dev, scheme, n;
     double h;
     bool operator<(const MKey &o) const {
-        return std::tie(dev, scheme, n, transposed, h) < std::tie(o.dev, o.scheme, o.n, o.transposed, o.h);
+        return std::tie(dev, scheme, n, h) < std::tie(o.dev, o.scheme, o.n, o.h);
     }
 };
 std::mutex g_m_mu;
 std::map<MKey, MmaTable> g_m_tables;   // entries and device buffers live until process exit; b null: none
 
-int build_mma(int scheme, int n, double h, double sign, bool transposed, MmaTable &t, std::vector<unsigned short> &b,
-              std::vector<double> &sigma) {
+int build_mma(int scheme, int n, double h, double sign, MmaTable &t, std::vector<unsigned short> &b) {
     const bool per = scheme == EMIX_SCHEME_BPER;
     t = MmaTable{};
     t.n = n;
@@ -724,23 +696,18 @@ int build_mma(int scheme, int n, double h, double sign, bool transposed, MmaTabl
     constexpr int cnt = kMmaWin * kMmaRows;
     std::vector<std::vector<real>> E((size_t)t.ntype * kMmaRows);
     real top = 0;
-    sigma.assign(transposed ? n : 0, 0.0);
     for (int ty = 0; ty < t.ntype; ++ty) {
         const bool mid = per || (ty == t.nlow && t.ntype > t.nlow + t.nhigh);
         const int blk = ty < t.nlow ? ty : t.nblk - (t.ntype - ty);
         for (int o = 0; o < kMmaRows; ++o) {
             std::vector<real> &e = E[(size_t)ty * kMmaRows + o];
             if (mid) {
-                inner.row(kMid + o, kMid - 40, cnt, e, false);
-                if (transposed)
-                    for (real &v : e) v = -v;   // without closures nearby D is antisymmetric
+                inner.row(kMid + o, kMid - 40, cnt, e);
             } else if (kMmaRows * blk + o < n) {
                 // differences before 0 and after n-2 do not exist; their columns stay zero
                 const int k0 = kMmaRows * blk - 40, ka = std::max(k0, 0), kb = std::min(k0 + cnt, n - 1);
                 std::vector<real> in;
-                const int i = kMmaRows * blk + o;
-                const real sum = own.row(i, ka, kb - ka, in, transposed);
-                if (transposed) sigma[i] = (double)(sum * (real)sign / (real)h);
+                own.row(kMmaRows * blk + o, ka, kb - ka, in);
                 e.assign(cnt, real(0));
                 for (int k = ka; k < kb; ++k) e[k - k0] = in[k - ka];
             } else {
@@ -803,34 +770,28 @@ int build_mma(int scheme, int n, double h, double sign, bool transposed, MmaTabl
 
 } // namespace
 
-int get_mma_table(int scheme, int n, double h, double sign, bool transposed, const MmaTable **out) {
+int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out) {
     *out = nullptr;
     if (n < kMmaMinN) return EMIX_OK;
     int dev = 0;
     EMIX_CUDA_TRY(cudaGetDevice(&dev));
-    MKey key{dev, scheme, n, transposed ? 1 : 0, sign * h};
+    MKey key{dev, scheme, n, sign * h};
     std::lock_guard<std::mutex> lock(g_m_mu);
     auto it = g_m_tables.find(key);
     if (it == g_m_tables.end()) {
         MmaTable t{};
         std::vector<unsigned short> b;
-        std::vector<double> sigma;
-        if (build_mma(scheme, n, h, sign, transposed, t, b, sigma)) {
+        if (build_mma(scheme, n, h, sign, t, b)) {
             t.b = nullptr;
         } else {
             void *buf = nullptr;
-            const size_t nb = b.size() * 2, ns = sigma.size() * sizeof(double);   // nb: whole types
-            if (cudaMalloc(&buf, nb + ns) != cudaSuccess) {
+            if (cudaMalloc(&buf, b.size() * 2) != cudaSuccess) {
                 cudaGetLastError();
                 set_last_message("cudaMalloc of a tensor-core derivative table failed");
                 return EMIX_ERR_ALLOC;
             }
-            EMIX_CUDA_TRY(cudaMemcpy(buf, b.data(), nb, cudaMemcpyHostToDevice));
+            EMIX_CUDA_TRY(cudaMemcpy(buf, b.data(), b.size() * 2, cudaMemcpyHostToDevice));
             t.b = (const unsigned short *)buf;
-            if (ns) {
-                EMIX_CUDA_TRY(cudaMemcpy((char *)buf + nb, sigma.data(), ns, cudaMemcpyHostToDevice));
-                t.sigma = (const double *)((char *)buf + nb);
-            }
         }
         it = g_m_tables.emplace(key, t).first;
     }
