@@ -4,48 +4,52 @@
 // The FP64 pipe (2 lanes per clock and SM) bounds the factored Thomas sweeps
 // at 3 clocks per cell and field.  Here D f is a contraction of the dense
 // operator, which falls off so fast that 96 differences reach 16 outputs
-// (deriv_mma.cuh), and its products are formed exactly on the tensor cores:
-// each pencil's differences are turned into fixed-point numbers (relative to
-// the pencil's largest difference) of six balanced digits to the base 1024,
-// the operator into digits of the same kind, and the f32 sums of digit
-// products are integers below 2^24 and so exact (the error-free splitting of
-// K. Ozaki et al., Numerical Algorithms 59, 2012, applied to a banded
-// operator).  Products of digit orders i + j <= 5 are kept; what is dropped
-// is 2^-57 of the largest term, an FP64 sum of the same terms rounds at
-// 2^-53.
+// (deriv_mma.cuh), and its products are formed on the tensor cores: each
+// pencil's differences are turned into fixed-point numbers (relative to the
+// pencil's largest difference, to 2^-60 of it) of six balanced digits to the base
+// 1024, the operator into digits of the same kind, and the sums of digit products
+// are integers in f32 (the error-free splitting of K. Ozaki et al., Numerical
+// Algorithms 59, 2012, applied to a banded operator).  Products of digit orders
+// i + j <= 5 are kept.
+//
+// Errors, relative to the pencil's largest difference over h: 2^-57 from the
+// products dropped, up to 2^-55.8 from the operator's cut at 40 rows.  The sweeps
+// err by a few 2^-53 of the differences nearby, so a pencil may be quiet nowhere:
+// one with a window of rows (16, along x 32) whose largest difference is below
+// 2^-kMmaSpan of the pencil's takes the sweep (deriv.cuh's arithmetic), and so do
+// infinities, NaN and magnitudes whose sums or results could leave the FP64 range.
+// A window's error is then at most 2^-45.5 of its largest difference over h, about
+// 2^-47 on average.  2^10: in a tank's first steps at 256^3 1 to 7% of the pencils
+// span more, 30 to 50% more than 2^8 and nearly all more than 2^4, since the walls'
+// no-slip jump is among them.  Over whole smooth fields the error against a dense
+// solve is no larger than the sweeps' (192 x 160 x 192, 2-norm: A 5.4e-15 ->
+// 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 -> 9.4e-16, C 5.7e-15 -> 3.4e-15).
 //
 // One CTA per SM walks tiles of 128 pencils (one per tensor-memory lane), its
 // warps in four roles that meet on mbarriers:
-//   three warps read the next tile once for each pencil's largest exponent and
-//     largest difference (the first tile is shared by all);
+//   seven warps read the next tile once for each pencil's largest difference and
+//     its quietest window's (the first tile is shared by all);
 //   eight warps convert the tile's differences to digits, 16 rows (a group) at
 //     a time, into tensor memory, where they are the instruction's A operand;
 //   one warp issues the products of a block of 16 outputs: 28 instructions,
 //     since the operator's digits 0 .. 5-j lie next to each other and one
 //     instruction adds all products of the differences' digit j;
 //   eight warps combine the finished block's six sums per output.
-// Whole tiles while they fill every SM, the rest cut into segments of blocks.
+// Whole tiles while they fill every SM, the rest cut into segments of blocks.  A
+// tile of which every pencil takes the sweep is left out of the last three roles;
+// the sweeps follow the CTA's last tile, a thread a pencil, or a warp if they are
+// few.
 //
-// What bounds it: the scanning warps (their loads come from DRAM, 12 KB in
-// flight per SM: a quarter of the scan took y from 0.514 to 0.434 ms) and the
-// tensor-core warp (28 instructions a block at 80 clocks each whatever their
-// width up to 128 columns; 16 outputs a block are what tensor memory holds
-// beside the digits) about alike, with the ALU pipe 55% busy (conversion 45
-// instructions a row, results 30, scan 11).  Two things made the issue of the
-// instructions cheap: elect.sync with warp-uniform operands (0.569 -> 0.522)
-// and a straight run of them, digit by digit, for the blocks whose six groups
-// all exist (-> 0.492).  More or fewer rows a scan step, L2 prefetch of the
-// rows to come, non-allocating loads and the scan spread over the other warps
-// (0.62) measured no better or worse.
-// Measured, ms for 5 fields of 256^3, sweeps -> here: closed x 1.001 -> 0.537,
-// y 0.991 -> 0.492, z 0.991 -> 0.498; cyclic 1.215 -> 0.557, 1.071 -> 0.567,
-// 1.069 -> 0.571.  Error against a dense solve, 192 x 160 x 192 smooth fields,
-// 2-norm: A 5.4e-15 -> 3.9e-15, B 1.2e-15 -> 1.1e-15, cyclic 9.8e-16 ->
-// 9.4e-16, C 5.7e-15 -> 3.4e-15.
-//
-// Pencils with infinities or NaN, or of magnitudes whose fixed-point
-// exponents would leave the FP64 range, take the scalar sweep (deriv.cuh)
-// after the tile.
+// What bounds it: the scanning warps (loads from DRAM, and the differences on the
+// FP64 pipe: 64 clocks of a quarter of the SM each) and the tensor-core warp (28
+// instructions a block at 80 clocks each whatever their width up to 128 columns;
+// 16 outputs a block are what tensor memory holds beside the digits) about alike,
+// with the ALU pipe 55% busy.  The instructions' operands stay in uniform registers
+// (elect.sync, branches on shuffled values): y 0.58 -> 0.52 ms.
+// Measured, ms for 5 fields of 256^3, sweeps -> here: closed x 1.001 -> 0.594,
+// y 0.993 -> 0.519, z 0.993 -> 0.522; cyclic 1.216 -> 0.631, 1.073 -> 0.580, 1.070
+// -> 0.583.  Where 1% of the pencils take the sweep x 0.64, y 0.58; 30% 1.16, 1.03;
+// all 2.05, 1.33.
 #include "deriv_mma.cuh"
 #include "tma.cuh"
 
@@ -62,9 +66,9 @@ __device__ int g_mma_timeouts = 0;
 
 constexpr int kMmaPencils = 128;            // per tile: the lanes of tensor memory
 constexpr int kRpt = 8;                     // rows of a group (outputs of a block) a thread takes at a time
-constexpr int kScanWarps = 3;               // warps that find the next tile's magnitudes
+constexpr int kScanWarps = 7;               // warps that find the next tile's magnitudes
 constexpr int kScan = 16;                   // rows a step of theirs
-constexpr int kScanParts = 4;               // parts a pencil (y, z) is scanned in
+constexpr int scan_parts(bool xax) { return xax ? 1 : 4; }   // parts a pencil is scanned in
 constexpr int kRole = 2 * kMmaPencils;      // converting threads, and as many for the results
 constexpr int kRoleWarps = kRole / 32;
 constexpr int kMmaThreads = 2 * kRole + 32 * (1 + kScanWarps);   // and the warp that drives the tensor core
@@ -93,6 +97,12 @@ int kind_of(int n, bool periodic) {
     return !periodic ? kClosed : (n % kMmaRows == 0 && n <= kMmaRoundN ? kRound : kCyclic);
 }
 constexpr int kMmaWaitNs = 10000, kMmaWaitLimit = 1 << 15;   // a wait's slices, and their number
+constexpr int kMmaSpan = 10;                // a window's largest difference to the pencil's, in powers of two
+constexpr int kMmaSweepJobs = 128;          // jobs of a CTA whose sweeps wait for its last tile
+// the sweeps a warp each where they are few: a warp takes 20 us for one at 256 rows,
+// 10 at 40, a thread 170 and 14
+constexpr int kSweepWarps = kMmaThreads / 32;
+constexpr int kMmaShared = 120 * 1024;      // least shared memory a CTA asks for
 constexpr int kXPitch = 17;                 // x pencils' staging tile: 17 rows, odd pitch
 constexpr int kXTileDoubles = kMmaPencils * kXPitch;
 static_assert(kLowCol + kLowRing * 24 <= kTmemCols, "tensor memory");
@@ -116,34 +126,29 @@ EMIX_DEV void tm_ld8(unsigned addr, float (&v)[8]) {
                  : "r"(addr));
 }
 
-// v 2^(62 - (E - 1023) + sh) modulo 2^64, truncated towards zero before the
-// shift by sh: below 2^61 in magnitude before it for E two above v's biased
-// exponent
-EMIX_DEV unsigned long long to_fixed(double v, int E, int sh) {
+// v 2^(62 - (E - 1023)) modulo 2^64, its magnitude truncated before a negative one's
+// bits are inverted: differences up to the biased exponent E come out below 2^63
+EMIX_DEV unsigned long long to_fixed(double v, int E) {
     const int hi = __double2hiint(v), lo = __double2loint(v);
-    const int r = E - ((hi >> 20) & 0x7ff);
+    const int up = ((hi >> 20) & 0x7ff) - E + 10;   // left shift of the mantissa
+    const int sl = max(up, 0), sr = max(-up, 0);
     const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const unsigned h = __funnelshift_l((unsigned)lo, mh, 10), l = (unsigned)lo << 10;
-    // 64-bit right shift: the funnel's shift is clamped at 32
+    // 64-bit shifts: a funnel's is clamped at 32
+    const unsigned h = __funnelshift_lc(0u, __funnelshift_lc((unsigned)lo, mh, sl), max(up - 32, 0));
+    const unsigned l = __funnelshift_lc(0u, (unsigned)lo, sl);
     const unsigned neg = (unsigned)(hi >> 31);
-    const unsigned rh = __funnelshift_rc(h, 0u, r) ^ neg;
-    const unsigned rl = __funnelshift_rc(__funnelshift_rc(l, h, r), 0u, max(r - 32, 0)) ^ neg;
-    const unsigned long long t = (((unsigned long long)rh << 32) | rl) + (neg & 1u);
-    return ((unsigned long long)__funnelshift_l((unsigned)t, (unsigned)(t >> 32), sh) << 32) | ((unsigned)t << sh);
+    const unsigned rh = __funnelshift_rc(h, 0u, sr) ^ neg;
+    const unsigned rl = __funnelshift_rc(__funnelshift_rc(l, h, sr), 0u, max(-32 - up, 0)) ^ neg;
+    return ((unsigned long long)rh << 32) | rl;
 }
 
-// a value's high word to about 20 bits as a float (2^-126 and less as 2^-126;
-// meaningful for values whose exponents fit)
-EMIX_DEV float rough(int hi) {
-    const unsigned t = (unsigned)max(hi & 0x7fffffff, 897 << 20) * 8u - (896u << 23);
-    return __uint_as_float((t & 0x7fffffffu) | ((unsigned)hi & 0x80000000u));
-}
-
-struct Spread {          // of one pencil, or a part of it
-    int top;             // largest |high word|
+// the differences of one pencil, or a part of it, by their high words without sign
+struct Spread {
+    int top;             // the largest
+    int least;           // of the windows' largest, the smallest
     unsigned low;        // low words, or-ed (zero test)
-    float diff;          // largest rough difference
 };
+EMIX_DEV int size_of(double d) { return __double2hiint(d) & 0x7fffffff; }
 
 // the ten-bit digits at bit P of two rows' words as two f16: the two bytes
 // they lie in, shifted down; 0x6400 | x is 1024 + x, and x carries a bias of 512
@@ -162,25 +167,214 @@ EMIX_DEV void digits(unsigned (&d)[kRpt / 2], const unsigned (&w)[kRpt]) {
     for (int q = 0; q < kRpt / 2; ++q) d[q] = digit_pair<P>(w[2 * q], w[2 * q + 1]);
 }
 
-// one pencil's magnitudes, once known: the exponent its values are fixed to,
-// the left shift of their differences, and whether it takes the scalar sweep
+// one pencil's magnitudes, once known: the exponent its differences are fixed to,
+// and whether it takes the scalar sweep: a window whose largest difference is below
+// 2^-kMmaSpan of the pencil's, infinities, NaN, and exponents whose sums or whose
+// results would leave the FP64 range
 struct Scale {
-    int E, sh;
+    int E;
     bool scalar;
 };
 
-EMIX_DEV Scale scale_of(const Spread &a) {
-    Scale r{1023, 0, false};
-    if (a.top == 0 && a.low == 0) return r;   // all zero
+EMIX_DEV Scale scale_of(const Spread &a, int se) {
+    Scale r{1023, false};
+    if (a.top == 0 && a.low == 0) return r;   // all alike
     const int e = a.top >> 20;
-    r.scalar = e < 256 || e > 1790;
-    r.E = e + 2;
-    if (e >= 930 && e <= 1140) {
-        // differences are below B: shift them up to 63 bits
-        const float B = fmaf(a.diff, 1.01f, __uint_as_float((unsigned)(e - 896 + 1 - 18) << 23));
-        r.sh = min(max(r.E - 1023 - ((int)(__float_as_uint(B) >> 23) - 127), 0), 25);
-    }
+    r.E = (a.top + 0x1000) >> 20;             // above 1 - 2^-8 of the next power of two: that one
+    r.scalar = e < 256 || e > 1790 || r.E - se < 16 || r.E - se > 1960 || a.top - a.least > kMmaSpan << 20;
     return r;
+}
+
+// D f (EPI_STORE) or out += D f (EPI_ACCUM) along one pencil, as deriv_pencil with
+// rows in runs of R: a run's loads are in flight while the one before it is walked.
+// Few warps sweep here, and a run of a row's neighbours along x shares its sectors.
+template <int EPI, bool PER>
+__device__ __noinline__ void sweep_pencil(const DerivTable &T, const double *__restrict__ in, double *w, double *out, long s) {
+    constexpr bool ACC = EPI == EPI_ACCUM;
+    constexpr int R = 8;
+    const int n = T.n;
+    const DerivRow *rows = T.rows;
+    const DerivRowU *ur = T.urows;
+    double up = 0.0, y0 = 0.0;
+    int i = 0;
+    auto closure = [&]() {
+        up = rhs_row(T, in, s, i) - (ACC ? __ldg(&ur[i].mu) : __ldg(&rows[i].m)) * up;
+        w[i * s] = up;
+    };
+    if (!PER)
+        for (; i < T.nlo; ++i) closure();
+    const int iend = PER ? n : n - T.nhi, ku = PER ? min(T.ku, n) : 0;
+    double fm2 = in[(PER ? n - 2 : i - 2) * s], fm1 = in[(PER ? n - 1 : i - 1) * s], f0 = in[i * s], fp1 = in[(i + 1) * s];
+    double nf[R];   // f(i + 2) of the next run's rows
+    auto fetch = [&](int b) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const int j = b + q + 2;
+            nf[q] = in[(PER ? (j >= n ? j - n : j) : min(j, n - 1)) * s];
+        }
+    };
+    fetch(i);
+    for (; i < iend; i += R) {
+        double f[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) f[q] = nf[q];
+        if (i + R < iend) fetch(i + R);
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const int k = i + q;
+            if (k >= iend) break;
+            const double fp2 = f[q];
+            double v;
+            if constexpr (ACC)
+                v = fma(__ldg(&ur[k].c), fp2 - fm2, fp1 - fm1) - __ldg(&ur[k].mu) * up;
+            else
+                v = __ldg(&rows[k].A) * (fp1 - fm1) + __ldg(&rows[k].B) * (fp2 - fm2) - __ldg(&rows[k].m) * up;
+            w[k * s] = v;
+            if (PER && k < ku) y0 += __ldg(ACC ? &T.u0s[k] : &T.u0[k]) * v;
+            up = v;
+            fm2 = fm1; fm1 = f0; f0 = fp1; fp1 = fp2;
+        }
+    }
+    if (!PER)
+        for (i = iend; i < n; ++i) closure();
+
+    const double fact = PER ? (y0 + (ACC ? T.sm1s : T.sm1) * up) * T.sm2 : 0.0;
+    double zn = 0.0, nw[R], no[R];
+    auto fetch_back = [&](int b) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            nw[q] = w[max(b - q, 0) * s];
+            if (ACC) no[q] = out[max(b - q, 0) * s];
+        }
+    };
+    fetch_back(n - 1);
+    for (i = n - 1; i >= 0; i -= R) {
+        double v[R], old[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            v[q] = nw[q];
+            if (ACC) old[q] = no[q];
+        }
+        if (i >= R) fetch_back(i - R);
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const int k = i - q;
+            if (k < 0) break;
+            zn = v[q] - __ldg(ACC ? &ur[k].gu : &rows[k].g) * zn;
+            const bool corr = PER && (k >= T.zhi || k < T.zlo);
+            if constexpr (ACC) {
+                double acc = old[q];
+                if (corr) acc -= fact * __ldg(&T.zz[k]);
+                out[k * s] = fma(__ldg(&ur[k].k), zn, acc);
+            } else {
+                out[k * s] = corr ? zn - fact * __ldg(&T.zz[k]) : zn;
+            }
+        }
+    }
+}
+
+// the same by one warp, a lane a run of rows: each recurrence is an affine map of
+// the value its lane starts from; the maps are composed by a scan and the runs
+// walked again from their values.  row: n doubles of the warp's own.  False (and
+// nothing stored) for infinities and NaN, which composed maps would spread.
+template <int EPI, bool PER>
+__device__ __noinline__ bool sweep_warp(const DerivTable &T, const double *__restrict__ in, double *out, long s,
+                                        double *row, int lane) {
+    constexpr bool ACC = EPI == EPI_ACCUM;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int n = T.n, R = ((n + 31) / 32) | 1;   // odd: no bank conflicts
+    const int first = min(lane * R, n), end = min(first + R, n);
+    const DerivRow *rows = T.rows;
+    const DerivRowU *ur = T.urows;
+    bool finite = true;
+    for (int i = lane; i < n; i += 32) {
+        const double f = in[i * s];
+        finite = finite && size_of(f) < 0x7ff00000;
+        row[i] = f;
+    }
+    if (!__all_sync(kAll, finite)) return false;
+    // what other runs hold, before they are overwritten
+    auto at = [&](int i) { return row[PER ? (i < 0 ? i + n : (i >= n ? i - n : i)) : min(max(i, 0), n - 1)]; };
+    double fm2 = at(first - 2), fm1 = at(first - 1), f0 = at(first), fp1 = at(first + 1);
+    const double e0 = at(end), e1 = at(end + 1);
+    double lo[4], hi[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        lo[q] = row[q];
+        hi[q] = row[n - 1 - q];
+    }
+    __syncwarp();
+    // right-hand sides, and each run from zero
+    double a = 1.0, b = 0.0;
+    for (int i = first; i < end; ++i) {
+        const double fp2 = i + 2 < end ? row[i + 2] : (i + 2 == end ? e0 : e1);
+        double r;
+        if (!PER && (i < T.nlo || i >= n - T.nhi)) {
+            const bool top = i >= T.nlo;
+            const double *c = top ? T.chi + 4 * (n - 1 - i) : T.clo + 4 * i;
+            r = c[0] * (top ? hi[0] : lo[0]) + c[1] * (top ? hi[1] : lo[1]) + c[2] * (top ? hi[2] : lo[2]) +
+                c[3] * (top ? hi[3] : lo[3]);
+        } else if constexpr (ACC) {
+            r = fma(__ldg(&ur[i].c), fp2 - fm2, fp1 - fm1);
+        } else {
+            r = __ldg(&rows[i].A) * (fp1 - fm1) + __ldg(&rows[i].B) * (fp2 - fm2);
+        }
+        const double m = ACC ? __ldg(&ur[i].mu) : __ldg(&rows[i].m);
+        b = r - m * b;
+        a *= -m;
+        row[i] = r;
+        fm2 = fm1; fm1 = f0; f0 = fp1; fp1 = fp2;
+    }
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const double pa = __shfl_up_sync(kAll, a, d), pb = __shfl_up_sync(kAll, b, d);
+        if (lane >= d) {
+            b = fma(a, pb, b);
+            a *= pa;
+        }
+    }
+    double v = __shfl_up_sync(kAll, b, 1), y0 = 0.0;
+    if (lane == 0) v = 0.0;
+    for (int i = first; i < end; ++i) {
+        v = row[i] - (ACC ? __ldg(&ur[i].mu) : __ldg(&rows[i].m)) * v;
+        row[i] = v;
+        if (PER && i < T.ku) y0 += __ldg(ACC ? &T.u0s[i] : &T.u0[i]) * v;
+    }
+    double fact = 0.0;
+    if constexpr (PER) {
+#pragma unroll
+        for (int d = 16; d; d /= 2) y0 += __shfl_xor_sync(kAll, y0, d);
+        fact = (y0 + (ACC ? T.sm1s : T.sm1) * __shfl_sync(kAll, v, (n - 1) / R)) * T.sm2;
+    }
+    a = 1.0;
+    b = 0.0;
+    for (int i = end - 1; i >= first; --i) {
+        const double g = ACC ? __ldg(&ur[i].gu) : __ldg(&rows[i].g);
+        b = row[i] - g * b;
+        a *= -g;
+    }
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const double pa = __shfl_down_sync(kAll, a, d), pb = __shfl_down_sync(kAll, b, d);
+        if (lane + d < 32) {
+            b = fma(a, pb, b);
+            a *= pa;
+        }
+    }
+    double z = __shfl_down_sync(kAll, b, 1);
+    if (lane == 31) z = 0.0;
+    for (int i = end - 1; i >= first; --i) {
+        z = row[i] - (ACC ? __ldg(&ur[i].gu) : __ldg(&rows[i].g)) * z;
+        row[i] = z;
+    }
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        const double corr = PER && (i >= T.zhi || i < T.zlo) ? fact * __ldg(&T.zz[i]) : 0.0;
+        if constexpr (ACC) out[i * s] = fma(__ldg(&ur[i].k), row[i], out[i * s] - corr);
+        else out[i * s] = row[i] - corr;
+    }
+    __syncwarp();
+    return true;
 }
 
 // a tile of pencils as one thread sees it
@@ -193,68 +387,71 @@ struct Tile {
     bool live;
 };
 
-// magnitudes of the 128 x pencils from p0 of field f: P at a time, lanes along
-// the rows, kScan / P rounds of 32 rows each (P = 1: as many as it takes)
+// magnitudes of the 128 x pencils from p0 of field f: P at a time, two rows a
+// lane, kScan / P / 2 rounds of 64 rows (two windows) each (P = 1: as many as it takes)
 template <int P, bool PER>
 EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, int lane, Spread *to) {
     constexpr int C = kScan / P;
+    constexpr bool kBefore = P == 1 || (PER && P <= 4);   // the value before the pencil: loaded, or among its rows
+    constexpr int kB = kBefore ? P : 1;
     const int steps = P == 1 ? (n + 32 * C - 1) / (32 * C) : 1;
-    double sv[kScan], before[P];
-    int top[P];
-    unsigned low[P];
-    float diff[P], prev[P];
+    double sv[kScan], before[kB], last = 0.0;   // last: P = 1, the rows' last value so far
+    int top = 0, least = 0;
+    unsigned low = 0;
     auto load = [&](int u, int st) {
-        const int r = st * 32 * C + lane;
+        const int r = st * 32 * C + 2 * lane;
 #pragma unroll
         for (int i = 0; i < P; ++i) {
             const double *fp = f + (long)min(p0 + u * P + i, np - 1) * n;
-            if (st == 0) before[i] = fp[PER ? n - 1 : 0];
+            if (kBefore && st == 0) before[i < kB ? i : 0] = fp[PER ? n - 1 : 0];
 #pragma unroll
-            for (int q = 0; q < C; ++q) sv[i * C + q] = fp[min(r + 32 * q, n - 1)];
+            for (int q = 0; q < C; ++q) sv[i * C + q] = fp[min(r + 64 * (q >> 1) + (q & 1), n - 1)];
         }
     };
     int u = uw, st = 0;
     if (u < kMmaPencils / P) load(u, 0);
     while (u < kMmaPencils / P) {
-        if (st == 0) {
 #pragma unroll
-            for (int i = 0; i < P; ++i) {
-                top[i] = 0;
-                low[i] = 0;
-                diff[i] = 0.0f;
-                prev[i] = rough(__double2hiint(before[i]));
+        for (int i = 0; i < P; ++i) {
+            if (st == 0) {
+                top = 0;
+                least = 0x7fffffff;
+                low = 0;
+                if constexpr (kBefore) last = before[i < kB ? i : 0];
+                else if constexpr (PER) {   // 64 rows at most
+                    const double x = __shfl_sync(0xffffffffu, sv[i * C], (n - 1) >> 1);
+                    last = __shfl_sync(0xffffffffu, sv[i * C + 1], (n - 1) >> 1);
+                    if ((n - 1) % 2 == 0) last = x;
+                } else {
+                    last = __shfl_sync(0xffffffffu, sv[i * C], 0);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < C; q += 2) {
+                const double x = sv[i * C + q], y = sv[i * C + q + 1];
+                const double d = x - __shfl_sync(0xffffffffu, lane == 31 ? last : y, (lane + 31) & 31), e = y - x;
+                last = y;
+                low |= (unsigned)__double2loint(d) | (unsigned)__double2loint(e);
+                const int m = max(size_of(d), size_of(e));
+                // the lower and the upper 16 lanes' rows
+                const int w0 = __reduce_max_sync(0xffffffffu, lane < 16 ? m : 0);
+                const int w1 = __reduce_max_sync(0xffffffffu, lane < 16 ? 0 : m);
+                top = max(top, max(w0, w1));
+                // the rows after the last whole window count with it
+                const int r = 32 * (st * C + q);
+                if (r + 32 <= n) least = min(least, w0);
+                if (r + 64 <= n) least = min(least, w1);
+            }
+            if (st == steps - 1) {
+                const unsigned lw = __reduce_or_sync(0xffffffffu, low);
+                if (lane == 0) to[u * P + i] = Spread{top, least, lw};
             }
         }
-        int hi[kScan];
-#pragma unroll
-        for (int q = 0; q < kScan; ++q) {
-            hi[q] = __double2hiint(sv[q]);
-            low[q / C] |= (unsigned)__double2loint(sv[q]);
-        }
-        const int uu = u;
         if (++st == steps) {
             st = 0;
             u += step;
         }
         if (u < kMmaPencils / P) load(u, st);
-#pragma unroll
-        for (int q = 0; q < kScan; ++q) {
-            const int i = q / C;
-            top[i] = max(top[i], hi[q] & 0x7fffffff);
-            const float x = rough(hi[q]);
-            const float pr = __shfl_sync(0xffffffffu, lane == 31 ? prev[i] : x, (lane + 31) & 31);
-            diff[i] = fmaxf(diff[i], fabsf(x - pr));
-            prev[i] = x;
-        }
-        if (u != uu) {
-#pragma unroll
-            for (int i = 0; i < P; ++i) {
-                const int tp = __reduce_max_sync(0xffffffffu, top[i]);
-                const unsigned lw = __reduce_or_sync(0xffffffffu, low[i]);
-                const unsigned d = __reduce_max_sync(0xffffffffu, __float_as_uint(diff[i]));   // not negative
-                if (lane == 0) to[uu * P + i] = Spread{tp, lw, __uint_as_float(d)};
-            }
-        }
     }
 }
 
@@ -264,6 +461,7 @@ EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, i
 template <bool XAX, int EPI, int KIND>
 EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     constexpr bool PER = KIND == kCyclic || KIND == kRound;
+    constexpr int kScanParts = scan_parts(XAX);
     const MmaTable &M = I.M;
     const PencilFields &F = I.F;
     const int np = I.np, ntile = I.ntile, nf = I.nf, whole = I.whole, segs = I.segs, nx = I.nx, ncta = I.ncta;
@@ -280,6 +478,8 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         s_scaled[2], s_read[2], s_table;
     __shared__ Spread s_part[2][kScanParts][kMmaPencils];   // by the tile's parity
     __shared__ unsigned char s_scalar[kMmaPencils];
+    __shared__ unsigned s_sweep[kMmaSweepJobs][4];   // pencils of the CTA's jobs that take the scalar sweep
+    __shared__ int s_sweeps;                          // their number
     const int tid = threadIdx.x, lane = tid & 31;
     // through a shuffle: the roles' branches are then known to be uniform, and
     // the instruction operands stay in uniform registers
@@ -288,11 +488,12 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
 
     if (tid == 0) {
         s_fail = 0;
+        s_sweeps = 0;
         for (int q = 0; q < 2; ++q) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_full[q])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_drained[q])), "r"(kRoleWarps) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_scaled[q])), "r"(kScanWarps) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_read[q])), "r"(2 * kRoleWarps) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_read[q])), "r"(2 * kRoleWarps + 1) : "memory");
         }
         for (int q = 0; q < 8; ++q) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&s_conv[q])), "r"(kRoleWarps) : "memory");
@@ -390,11 +591,12 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         if constexpr (!XAX) {
             // units of 32 pencils (lanes) by a part of the rows
             const int part = (n + kScanParts - 1) / kScanParts, steps = (part + kScan - 1) / kScan;
-            double sv[kScan], before = 0.0;    // before: the value before the unit's first row
+            double sv[kScan], before = 0.0, prev = 0.0;   // before: the value before the unit's first row
             const double *fp = nullptr;
-            int ra = 0, rb = 0, top = 0;
+            int ra = 0, rb = 0, top = 0, least = 0;
             unsigned low = 0;
-            float diff = 0.0f, prev = 0.0f;
+            int rows = 0;                      // rows loaded that are the part's
+            bool window = false;               // they are one that counts by itself
             auto load = [&](int u, int st) {
                 if (st == 0) {
                     fp = tile_of(job, (u & 3) * 32 + lane).in;
@@ -404,6 +606,9 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                 }
                 const int r = ra + st * kScan;
                 const double *q0 = fp + (long)r * s;
+                // fewer rows count with the window before them
+                rows = min(kScan, rb - r + 1);
+                window = rows == kScan || st == 0;
                 if (r + kScan <= n) {
 #pragma unroll
                     for (int q = 0; q < kScan; ++q) sv[q] = q0[q * s];
@@ -417,30 +622,28 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             while (u < 4 * kScanParts) {
                 if (st == 0) {
                     top = 0;
+                    least = 0x7fffffff;
                     low = 0;
-                    diff = 0.0f;
-                    prev = rough(__double2hiint(before));
+                    prev = before;
                 }
-                int hi[kScan];
+                int w = 0;
 #pragma unroll
                 for (int q = 0; q < kScan; ++q) {
-                    hi[q] = __double2hiint(sv[q]);
-                    low |= (unsigned)__double2loint(sv[q]);
+                    if (q >= rows) break;
+                    const double d = sv[q] - prev;
+                    prev = sv[q];
+                    w = max(w, size_of(d));
+                    low |= (unsigned)__double2loint(d);
                 }
+                top = max(top, w);
+                if (window) least = min(least, w);
                 const int uu = u;
                 if (++st == steps) {
                     st = 0;
                     u += step;
                 }
                 if (u < 4 * kScanParts) load(u, st);
-#pragma unroll
-                for (int q = 0; q < kScan; ++q) {
-                    top = max(top, hi[q] & 0x7fffffff);
-                    const float x = rough(hi[q]);
-                    diff = fmaxf(diff, fabsf(x - prev));
-                    prev = x;
-                }
-                if (u != uu) s_part[buf][uu >> 2][(uu & 3) * 32 + lane] = Spread{top, low, diff};
+                if (u != uu) s_part[buf][uu >> 2][(uu & 3) * 32 + lane] = Spread{top, least, low};
             }
         } else {
             const Tile tl = tile_of(job, 0);
@@ -450,6 +653,36 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             else if (n <= 32 * (kScan / 2)) scan_x<2, PER>(tl.in, tl.p0, np, n, uw, step, lane, to);
             else scan_x<1, PER>(tl.in, tl.p0, np, n, uw, step, lane, to);
         }
+    };
+    // slot's pencil of tile t (from p0), once its magnitudes are known; skip: every
+    // pencil of the tile takes the sweep, and the roles leave it out
+    auto scale_wait = [&](int t, int p0, int slot, bool &skip) {
+        if (t > 0) wait(&s_scaled[t & 1], (unsigned)((t - 1) >> 1) & 1);
+        auto scale = [&](int q) {
+            Spread a = s_part[t & 1][0][q];
+#pragma unroll
+            for (int i = 1; i < kScanParts; ++i) {
+                const Spread b = s_part[t & 1][i][q];
+                a.top = max(a.top, b.top);
+                a.least = min(a.least, b.least);
+                a.low |= b.low;
+            }
+            return scale_of(a, M.se);
+        };
+        const Scale sc = scale(slot);
+        bool all = __all_sync(0xffffffffu, sc.scalar || p0 + slot >= np);
+#pragma unroll 1
+        for (int q = lane; q < kMmaPencils && all; q += 32)
+            all = __all_sync(0xffffffffu, scale(q).scalar || p0 + q >= np);
+        skip = __shfl_sync(0xffffffffu, (int)all, 0);   // known to be uniform
+        arrive(&s_read[t & 1]);
+        return sc;
+    };
+    // the sweep of the caller's pencil of a tile
+    auto sweep = [&](const Tile &t) {
+        const long x = XAX ? t.wofs : 0;
+        double *w = pick(F.w, t.field) + t.wofs;
+        sweep_pencil<EPI, PER>(I.T, t.in + x, w, t.out + x, s);
     };
     constexpr int kPencilWarps = 2 * kRoleWarps + kScanWarps;   // all but the tensor core's
     wait_for_previous();   // what is read so far is constant
@@ -471,8 +704,12 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             int B = 0, first = 0;     // block, and the tile's first group, counted over the tiles
             int seen = 0;             // groups known to be in tensor memory
             wait(&s_table, 0);
-            for (int job = cta; job < jobs; job += ncta) {
+            int t = 0;
+            for (int job = cta; job < jobs; job += ncta, ++t) {
                 const Tile jt = tile_of(job, 0);
+                bool skip;
+                scale_wait(t, jt.p0, lane, skip);
+                if (skip) continue;
                 for (int b = jt.b0; b < jt.b1; ++b, ++B) {
                     for (const int need = first + min(b + 3, jt.gb) - jt.ga; seen <= need; ++seen)
                         wait(&s_conv[seen & 7], (unsigned)(seen >> 3) & 1);
@@ -553,22 +790,6 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
         const unsigned tml = tm + ((unsigned)(quarter * 32) << 16);
         double *xin = reinterpret_cast<double *>(dyn + (size_t)M.ntype * kMmaTypeBytes);
         double *xout = xin + 2 * kXTileDoubles;
-        // this thread's pencil of tile t, once its magnitudes are known
-        auto scale_wait = [&](int t) {
-            if (t > 0) wait(&s_scaled[t & 1], (unsigned)((t - 1) >> 1) & 1);
-            Spread a = s_part[t & 1][0][slot_p];
-            if constexpr (!XAX) {
-#pragma unroll
-                for (int q = 1; q < kScanParts; ++q) {
-                    const Spread b = s_part[t & 1][q][slot_p];
-                    a.top = max(a.top, b.top);
-                    a.low |= b.low;
-                    a.diff = fmaxf(a.diff, b.diff);
-                }
-            }
-            arrive(&s_read[t & 1]);
-            return scale_of(a);
-        };
         if (!results) {
             // ---- a group's rows to digits, loaded one group ahead ---------------
             double v[kRpt + 1];   // y, z: the thread's rows; x: staged values
@@ -612,10 +833,10 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             auto convert = [&](int c, const Scale &sc) {
                 unsigned w1[kRpt], w2[kRpt];
                 const double *t = xin + (c & 1) * kXTileDoubles + slot_p * kXPitch + kRpt * rg;
-                unsigned long long a = to_fixed(XAX ? t[0] : v[0], sc.E, sc.sh);
+                unsigned long long a = to_fixed(XAX ? t[0] : v[0], sc.E);
 #pragma unroll
                 for (int q = 0; q < kRpt; ++q) {
-                    const unsigned long long b = to_fixed(XAX ? t[q + 1] : v[q + 1], sc.E, sc.sh);
+                    const unsigned long long b = to_fixed(XAX ? t[q + 1] : v[q + 1], sc.E);
                     // digits at bits 4 + 10 j, biased by 512; half of the bits dropped below
                     const unsigned long long y = b - a + 0x8020080200802008ull;
                     a = b;
@@ -649,17 +870,27 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                 if (round) reach = nblk;
                 if (pos >= 0) return B + min(cur.ga + pos + reach, cur.b1 - 1) - cur.b0;
                 const int Bl = B - (last.b1 - last.b0);
-                if (t == 0) return -1;
+                if (!B) return -1;
                 pos += last.gb - last.ga + 1;
                 return pos >= 0 ? Bl + min(last.ga + pos + reach, last.b1 - 1) - last.b0 : Bl - 1;
             };
             load(cur, cur.ga);
             for (; job < jobs; job += ncta, ++t) {
-                const Scale sc = scale_wait(t);
+                bool skip;
+                const Scale sc = scale_wait(t, cur.p0, slot_p, skip);
                 const bool more = job + ncta < jobs;
                 Tile nxt = cur;
                 if (more) nxt = tile_of(job + ncta, slot_p);
                 const int ng = cur.gb - cur.ga + 1;
+                if (skip) {
+                    // (as many barriers as of other tiles: a wait that ran out may have
+                    // left the warps of different minds)
+                    if constexpr (XAX)
+                        for (int k = 0; k < ng; ++k) row_sync(1);
+                    if (more) load(nxt, nxt.ga);
+                    cur = nxt;
+                    continue;
+                }
                 for (int k = 0; k < ng; ++k, ++c) {
                     // the rings' places are free once the blocks that read them are done
                     const int need = max(last_use(k - kHighRing, 2), last_use(k - kLowRing, 1));
@@ -703,9 +934,26 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             int B = 0, t = 0;
             for (int job = cta; job < jobs; job += ncta, ++t) {
                 const Tile cur = tile_of(job, slot_p);
-                const Scale sc = scale_wait(t);
-                const int escale = (sc.E - 1023 - M.se - sc.sh) * (1 << 20);
+                bool skip;
+                const Scale sc = scale_wait(t, cur.p0, slot_p, skip);
+                const int escale = (sc.E - 1023 - M.se) * (1 << 20);
                 if (XAX && rg == 0) s_scalar[slot_p] = sc.scalar;
+                // the pencils that take the sweep: after the tiles, by all warps
+                // (those of jobs past the record's end: now)
+                if (rg == 0) {
+                    const bool mine = sc.scalar && cur.live && ok && cur.b0 == 0;
+                    const unsigned m = __ballot_sync(0xffffffffu, mine);
+                    if (t < kMmaSweepJobs) {
+                        if (lane == 0) s_sweep[t][quarter] = m;
+                    } else if (mine) {
+                        sweep(cur);
+                    }
+                }
+                if (skip) {
+                    if constexpr (XAX)
+                        for (int q = (cur.b1 - cur.b0) * (3 - kOutTiles); q >= 0; --q) row_sync(2);
+                    continue;
+                }
                 for (int b = cur.b0; b < cur.b1; ++b, ++B) {
                     const int row = kMmaRows * b + kRpt * rg;
                     double old[kRpt];
@@ -767,12 +1015,6 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                         if constexpr (kOutTiles == 1) row_sync(2);   // the tile is free
                     }
                 }
-                // the pencils outside the fixed-point range
-                if (rg == 0 && sc.scalar && cur.live && ok && cur.b0 == 0) {
-                    const long x = XAX ? cur.wofs : 0;
-                    double *w = pick(F.w, cur.field) + cur.wofs;
-                    deriv_pencil<EPI>(I.T, cur.in + x, w, cur.out + x, s);
-                }
                 if constexpr (XAX) row_sync(2);   // s_scalar is free
             }
         }
@@ -787,6 +1029,32 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tm), "r"(kTmemCols));
+    // the sweeps: their list, then a row buffer for each warp, in dyn, which nothing
+    // reads any more
+    static_assert(kMmaSweepJobs * 4 <= kMmaThreads && kMmaSweepJobs * kMmaPencils <= 65536, "s_sweep");
+    const int mine = (jobs - cta + ncta - 1) / ncta;
+    unsigned bits = tid < 4 * min(mine, kMmaSweepJobs) && !s_fail ? s_sweep[tid >> 2][tid & 3] : 0;
+    if (!__syncthreads_or(bits != 0)) return;
+    unsigned short *list = reinterpret_cast<unsigned short *>(dyn);
+    if (bits) {
+        int at = atomicAdd(&s_sweeps, __popc(bits));
+        for (; bits; bits &= bits - 1) list[at++] = (unsigned short)(32 * tid + __ffs((int)bits) - 1);
+    }
+    __syncthreads();
+    const int count = s_sweeps;
+    if (count > kSweepWarps * max(1, n / 96)) {
+        for (int q = tid; q < count; q += kMmaThreads) sweep(tile_of(cta + (list[q] >> 7) * ncta, list[q] & 127));
+        return;
+    }
+    constexpr int kListBytes = kSweepWarps * (kTableMaxN / 96) * 2;
+    const int warps = min((kMmaShared - kListBytes) / (8 * n), kSweepWarps);
+    if (warp >= warps) return;
+    double *row = reinterpret_cast<double *>(dyn + kListBytes) + (size_t)warp * n;
+    for (int q = warp; q < count; q += warps) {
+        const Tile t = tile_of(cta + (list[q] >> 7) * ncta, list[q] & 127);
+        const long x = XAX ? t.wofs : 0;
+        if (!sweep_warp<EPI, PER>(I.T, t.in + x, t.out + x, s, row, lane) && lane == 0) sweep(t);
+    }
 }
 
 template <bool XAX, int EPI, int KIND>
@@ -815,7 +1083,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaIte
 template <bool XAX, int KIND>
 int shared_bytes(int ntype) {
     const int shm = ntype * kMmaTypeBytes + (XAX ? (2 + out_tiles(KIND)) * kXTileDoubles * (int)sizeof(double) : 0);
-    return shm < 120 * 1024 ? 120 * 1024 : shm;
+    return shm < kMmaShared ? kMmaShared : shm;
 }
 
 // divides item I between at most `n` CTAs (I.ncta: those that get work):

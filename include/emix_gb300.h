@@ -6,8 +6,10 @@
  * types.  Fields are Fortran column-major (i fastest, index
  * i + nx*(j + ny*k)); multi-component arrays stack components with stride
  * nx*ny*nz.  All values are IEEE FP64; derivatives along axes of 40 rows and
- * more are exact sums of integer digit products on the tensor cores, rounded to
- * FP64 with the error of an FP64 solve or less.
+ * more are sums of integer digit products on the tensor cores, within 2^-55 of a
+ * pencil's largest difference over the spacing (in the norm of a smooth pencil no
+ * more than an FP64 solve's error).  Pencils in which some 32 rows differ by less
+ * than 2^-10 of that, and infinities and NaN, are solved in FP64.
  *
  * Two families of entry points:
  *   - the reference's own symbols (cudaDeriv, cuDivergence) with byte-identical
