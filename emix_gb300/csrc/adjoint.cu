@@ -17,6 +17,7 @@
 #include "adjoint.cuh"
 #include "adjoint_weno.cuh"
 #include "ctx.cuh"
+#include "deriv_mma.cuh"
 
 #include <cstring>
 #include <new>
@@ -35,6 +36,7 @@ struct emix_adj {
     emix_ctx *c = nullptr;
     int nsteps = 0, every = 1;
     bool keep = false;               // every = 0: every step's tape kept, no recomputation
+    emix::TimeoutWatch watch;        // of the forward or the reverse sweep
     emix_objective obj{};
     double *arena = nullptr;
     size_t bytes = 0;
@@ -557,7 +559,8 @@ int emix_adj_device_bytes(emix_adj *a, size_t *bytes) {
 
 int emix_adj_forward(emix_adj *a, double *J) {
     if (!a || !J) return EMIX_ERR_ARG;
-    int rc;
+    int rc = a->watch.begin(a->c->stream);
+    if (rc) return rc;
     if (a->keep) {
         // every step taped as it runs: the reverse sweep recomputes nothing
         emix_ctx *c = a->c;
@@ -568,9 +571,10 @@ int emix_adj_forward(emix_adj *a, double *J) {
         }
         if ((rc = copy(a->final_clock_full, c->clock, kImpClockLen, c->stream))) return rc;
         if ((rc = save_state(a, a->final_state, a->final_clock))) return rc;
-        if ((rc = objective(a, false, J))) return rc;
+        if ((rc = a->watch.end(c->stream))) return rc;
+        if ((rc = objective(a, false, J))) return rc;   // synchronises
         a->J = *J;
-        return EMIX_OK;
+        return a->watch.result("emix_adj_forward");
     }
     // checkpoints every `every` steps from the context's current state
     for (int k = 0; k < a->nsteps; k += a->every) {
@@ -580,16 +584,18 @@ int emix_adj_forward(emix_adj *a, double *J) {
         if ((rc = run_steps(a, m, nullptr, nullptr, 0))) return rc;
     }
     if ((rc = save_state(a, a->final_state, a->final_clock))) return rc;
-    if ((rc = objective(a, false, J))) return rc;
+    if ((rc = a->watch.end(a->c->stream))) return rc;
+    if ((rc = objective(a, false, J))) return rc;   // synchronises
     a->J = *J;
-    return EMIX_OK;
+    return a->watch.result("emix_adj_forward");
 }
 
 int emix_adj_backward(emix_adj *a, double *dJ) {
     if (!a || !dJ) return EMIX_ERR_ARG;
     emix_ctx *c = a->c;
     const long n = c->n;
-    int rc;
+    int rc = a->watch.begin(c->stream);
+    if (rc) return rc;
     const long step_index = c->step_index;   // the recomputations below advance it
     if ((rc = zero(a->red, 2, c->stream))) return rc;
     // adjoint of J at the final state: a->LA (um0), a->Lphi (phi)
@@ -624,6 +630,7 @@ int emix_adj_backward(emix_adj *a, double *dJ) {
             t = a->Lphi; a->Lphi = a->Lphi_prev; a->Lphi_prev = t;
         }
     }
+    if ((rc = a->watch.end(c->stream))) return rc;
     double h[3];
     EMIX_CUDA_TRY(cudaMemcpyAsync(h, a->red, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     EMIX_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -632,7 +639,7 @@ int emix_adj_backward(emix_adj *a, double *dJ) {
     // leave the context at the final state of the forward pass
     if ((rc = load_state(a, a->final_state, a->final_clock))) return rc;
     c->step_index = step_index;
-    return EMIX_OK;
+    return a->watch.result("emix_adj_backward");
 }
 
 int emix_adj_state_gradient(emix_adj *a, double *lum, double *lphi) {

@@ -56,6 +56,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cstdio>
 #include <type_traits>
 #include <vector>
 
@@ -63,6 +64,7 @@ namespace emix {
 namespace {
 
 __device__ int g_mma_timeouts = 0;
+__device__ int g_mma_drop = 0;              // test hook: finished blocks are not signalled
 
 constexpr int kMmaPencils = 128;            // per tile: the lanes of tensor memory
 constexpr int kRpt = 8;                     // rows of a group (outputs of a block) a thread takes at a time
@@ -703,6 +705,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
             asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
             int B = 0, first = 0;     // block, and the tile's first group, counted over the tiles
             int seen = 0;             // groups known to be in tensor memory
+            const bool signal = leader && !*(volatile int *)&g_mma_drop;
             wait(&s_table, 0);
             int t = 0;
             for (int job = cta; job < jobs; job += ncta, ++t) {
@@ -764,7 +767,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                         }
                     }
                     __syncwarp();
-                    if (leader)
+                    if (signal)
                         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
                                      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];"
                                      :: "r"(smem_u32(&s_full[B & 1])), "r"(smem_u32(&s_done[B & 7])) : "memory");
@@ -1198,4 +1201,37 @@ int deriv_mma_timeouts(int *count) {
     return EMIX_OK;
 }
 
+int TimeoutWatch::note(int at, cudaStream_t st) {
+    if (!h_) {
+        if (cudaHostAlloc((void **)&h_, 4 * sizeof(int), cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            h_ = nullptr;
+            set_last_message("cudaHostAlloc of the timeout counters failed");
+            return EMIX_ERR_ALLOC;
+        }
+    }
+    EMIX_CUDA_TRY(cudaMemcpyFromSymbolAsync(h_ + at, g_mma_timeouts, sizeof(int), 0, cudaMemcpyDeviceToHost, st));
+    return pencil_tma_timeouts_async(h_ + at + 1, st);
+}
+
+int TimeoutWatch::result(const char *call) const {
+    if (h_[2] == h_[0] && h_[3] == h_[1]) return EMIX_OK;
+    char text[160];
+    snprintf(text, sizeof text, "%s: pencil blocks gave up waiting for the tensor core or for TMA row copies; its results "
+             "are incomplete", call);
+    set_last_message(text);
+    return EMIX_ERR_TIMEOUT;
+}
+
+TimeoutWatch::~TimeoutWatch() {
+    if (h_) cudaFreeHost(h_);
+}
+
 } // namespace emix
+
+extern "C" int emix_deriv_mma_test_drop(int on) {
+    if (on != 0 && on != 1) return EMIX_ERR_ARG;
+    EMIX_CUDA_TRY(cudaMemcpyToSymbol(emix::g_mma_drop, &on, sizeof(int)));
+    EMIX_CUDA_TRY(cudaDeviceSynchronize());
+    return EMIX_OK;
+}

@@ -91,5 +91,25 @@ int launch_deriv_mma_batch(const MmaBatch &b, bool xax, int epi, bool periodic, 
 
 // blocks that gave up a bounded wait since the library was loaded
 int deriv_mma_timeouts(int *count);
+// the sweeps' counter, copied on a stream (deriv_tma.cu)
+int pencil_tma_timeouts_async(int *count, cudaStream_t st);
+
+// Whether pencil blocks gave up a wait between two points of a stream's work: the
+// counters are copied at both, and read once the caller has synchronised.  (Blocks of
+// other streams' launches meanwhile count too.)
+class TimeoutWatch {
+public:
+    TimeoutWatch() = default;
+    TimeoutWatch(const TimeoutWatch &) = delete;
+    TimeoutWatch &operator=(const TimeoutWatch &) = delete;
+    ~TimeoutWatch();
+    int begin(cudaStream_t st) { return note(0, st); }
+    int end(cudaStream_t st) { return note(2, st); }
+    int result(const char *call) const;   // EMIX_OK or EMIX_ERR_TIMEOUT
+
+private:
+    int note(int at, cudaStream_t st);
+    int *h_ = nullptr;                    // pinned: tensor core and TMA, at the beginning and at the end
+};
 
 } // namespace emix

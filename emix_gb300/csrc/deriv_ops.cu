@@ -290,11 +290,12 @@ struct HostWs {
     double *buf[8] = {nullptr};
     size_t cap[8] = {0};
     cudaStream_t st[8] = {nullptr};
+    TimeoutWatch *watch[8] = {nullptr};   // (with the buffers: for the life of the process)
 };
 HostWs g_ws;
 int g_legacy_scheme = EMIX_SCHEME_C;
 
-int ws_get(size_t bytes, double **out, cudaStream_t *st) {
+int ws_get(size_t bytes, double **out, cudaStream_t *st, TimeoutWatch **watch) {
     int dev = 0;
     EMIX_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 8) return EMIX_ERR_ARG;
@@ -310,8 +311,10 @@ int ws_get(size_t bytes, double **out, cudaStream_t *st) {
         }
         g_ws.cap[dev] = bytes;
     }
+    if (!g_ws.watch[dev]) g_ws.watch[dev] = new TimeoutWatch;
     *out = g_ws.buf[dev];
     *st = g_ws.st[dev];
+    *watch = g_ws.watch[dev];
     return EMIX_OK;
 }
 } // namespace
@@ -408,18 +411,21 @@ int emix_cudaDeriv(const int schemes[3], double *dVel, double *dTemp, const doub
     const size_t n = ncell(nx, ny, nz);
     double *d;
     cudaStream_t st;
-    int rc = ws_get(16 * n * sizeof(double), &d, &st);
+    TimeoutWatch *watch;
+    int rc = ws_get(16 * n * sizeof(double), &d, &st, &watch);
     if (rc) return rc;
+    if ((rc = watch->begin(st))) return rc;
     double *dv = d, *dtp = d + 3 * n, *ddv = d + 4 * n, *ddt = d + 13 * n;
     EMIX_CUDA_TRY(cudaMemcpyAsync(dv, vel, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
     EMIX_CUDA_TRY(cudaMemcpyAsync(dtp, temp, n * sizeof(double), cudaMemcpyHostToDevice, st));
     const double h[3] = {hx, hy, hz};
     rc = cudaDeriv_dev_impl(schemes, ddv, ddt, dv, dtp, h, nx, ny, nz, st);
     if (rc) return rc;
+    if ((rc = watch->end(st))) return rc;
     EMIX_CUDA_TRY(cudaMemcpyAsync(dVel, ddv, 9 * n * sizeof(double), cudaMemcpyDeviceToHost, st));
     EMIX_CUDA_TRY(cudaMemcpyAsync(dTemp, ddt, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, st));
     EMIX_CUDA_TRY(cudaStreamSynchronize(st));
-    return EMIX_OK;
+    return watch->result("emix_cudaDeriv");
 }
 
 int emix_cuDivergence_dev(const int schemes[3], double *rs, double *rsv, const double *e,
@@ -454,8 +460,10 @@ int emix_cuDivergence(const int schemes[3], double *rs, double *rsv, const doubl
     double *d;
     cudaStream_t st;
     // inputs 6 + jbn 11 + outputs 2 + scratch 8
-    int rc = ws_get(27 * n * sizeof(double), &d, &st);
+    TimeoutWatch *watch;
+    int rc = ws_get(27 * n * sizeof(double), &d, &st, &watch);
     if (rc) return rc;
+    if ((rc = watch->begin(st))) return rc;
     double *de = d, *dj = d + 6 * n, *drs = d + 17 * n, *drsv = d + 18 * n, *scr = d + 19 * n;
     const double *src[6] = {e, f, g, ev, fv, gv};
     for (int q = 0; q < 6; ++q)
@@ -467,10 +475,11 @@ int emix_cuDivergence(const int schemes[3], double *rs, double *rsv, const doubl
     rc = cuDivergence_dev_impl(schemes, drs, drsv, de, de + n, de + 2 * n, de + 3 * n, de + 4 * n,
                                de + 5 * n, dj, h, nx, ny, nz, st, scr);
     if (rc) return rc;
+    if ((rc = watch->end(st))) return rc;
     EMIX_CUDA_TRY(cudaMemcpyAsync(rs, drs, n * sizeof(double), cudaMemcpyDeviceToHost, st));
     EMIX_CUDA_TRY(cudaMemcpyAsync(rsv, drsv, n * sizeof(double), cudaMemcpyDeviceToHost, st));
     EMIX_CUDA_TRY(cudaStreamSynchronize(st));
-    return EMIX_OK;
+    return watch->result("emix_cuDivergence");
 }
 
 void cudaDeriv(double *dVel, double *dTemp, double *vel, double *temp, double *amut,

@@ -583,6 +583,11 @@ int launch_deriv_t_yz_tma(const DerivTTable &T, const PencilMaps &M, int acc, in
 
 using namespace emix;
 
+int emix::pencil_tma_timeouts_async(int *count, cudaStream_t st) {
+    EMIX_CUDA_TRY(cudaMemcpyFromSymbolAsync(count, g_pencil_tma_timeouts, sizeof(int), 0, cudaMemcpyDeviceToHost, st));
+    return EMIX_OK;
+}
+
 extern "C" int emix_pencil_tma_timeouts(int *count) {
     if (!count) return EMIX_ERR_ARG;
     int mma = 0;

@@ -107,7 +107,9 @@ int emix_deriv_dev(int scheme, int axis, int nf, double *out, const double *in,
 int emix_deriv_pcr_dev(int scheme, int axis, int nf, double *out, const double *in, double h,
                        int steps, int nx, int ny, int nz, void *stream);
 
-/* cudaDeriv with status, explicit per-axis schemes, host pointers. */
+/* cudaDeriv with status, explicit per-axis schemes, host pointers.
+ * EMIX_ERR_TIMEOUT (here and from emix_cuDivergence) when a pencil block gave
+ * up a bounded wait meanwhile: the results are then incomplete. */
 int emix_cudaDeriv(const int schemes[3], double *dVel, double *dTemp,
                    const double *vel, const double *temp,
                    double hx, double hy, double hz, int nx, int ny, int nz);
@@ -425,6 +427,12 @@ int emix_pencil_tma_timeouts(int *count);
  * production run. */
 int emix_pencil_tma_test_drop(int on);
 
+/* The same for the tensor-core derivatives: 1 makes their launches signal no
+ * finished block (current device), so every block gives up after its wait
+ * (about 0.3 s), counts itself and stores nothing; 0 restores normal
+ * operation.  Never set in a production run. */
+int emix_deriv_mma_test_drop(int on);
+
 /* Test hook for the bounded waits: 1 makes the TMA level-set stages issue no
  * plane copies (current device), so every stage block gives up after its
  * waits (about a second), counts itself and leaves its cells unwritten; the
@@ -468,9 +476,10 @@ int emix_ctx_get_time(emix_ctx *ctx, double *t);
  * last RK update); page-locked host buffers let them run asynchronously.  The
  * values are those of emix_step, bit for bit.  Returns EMIX_ERR_TIMEOUT when
  * a level-set stage block or a y/z pencil block gave up waiting for its TMA
- * copies during the call (its cells are then unwritten).  emix_step and the
- * other device-pointer forms return before their kernels finish: their
- * callers poll emix_weno_tma_timeouts and emix_pencil_tma_timeouts instead. */
+ * copies, or a pencil block for the tensor core, during the call (its cells
+ * are then unwritten).  emix_step, emix_batch_step and the other device-pointer
+ * forms return before their kernels finish: their callers poll
+ * emix_weno_tma_timeouts and emix_pencil_tma_timeouts instead. */
 int emix_step_host(emix_ctx *ctx, double *um, double *phi, int nsteps);
 
 /* Number of kernel launches one step issues (for accounting; the records
@@ -604,7 +613,9 @@ int emix_adj_device_bytes(emix_adj *adj, size_t *bytes);
  * for bit either way. */
 int emix_adj_set_overlap(emix_adj *adj, int on);
 
-/* Run nsteps from the context's current state, keeping checkpoints; J out. */
+/* Run nsteps from the context's current state, keeping checkpoints; J out.
+ * EMIX_ERR_TIMEOUT (here and from emix_adj_backward) when a pencil block gave
+ * up a bounded wait meanwhile: the results are then incomplete. */
 int emix_adj_forward(emix_adj *adj, double *J);
 
 /* Reverse sweep after emix_adj_forward: dJ[0] = dJ/d(impeller omega),
