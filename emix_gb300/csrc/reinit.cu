@@ -243,6 +243,71 @@ __global__ void __launch_bounds__(kNT, 3) k_reinit_stage(const ReinitArgs a) {
     }
 }
 
+// The stage by cells, each with differences, metric pairs and sign of its own: 280
+// FP64 operations, two fields of scratch, any extent.
+__global__ void __launch_bounds__(256) k_reinit_cells(const ReinitArgs a, const double *__restrict__ jbn, double sx, double sy,
+                                                      double sz) {
+    const int nxg = a.nxg, nyg = a.nyg, nzg = a.nzg;
+    const long sxy = (long)nxg * nyg, ng = sxy * nzg;
+    for (long id = blockIdx.x * (long)blockDim.x + threadIdx.x; id < ng; id += (long)gridDim.x * blockDim.x) {
+        int c3[3];
+        cell_of(id, ng, nxg, nyg, c3[0], c3[1], c3[2]);
+        const int L3[3] = {nxg, nyg, nzg};
+        const long s3[3] = {1, nxg, sxy};
+        const double sc[3] = {sx, sy, sz};
+        const double p0 = a.phi[id];
+        const int tsg = (p0 > 0.0) - (p0 < 0.0);
+        double r = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double C = sc[d] * jbn[4 * d * ng + id];
+            const double eps = kWenoEps4 * rcp_fast(C * C);
+            const long s = s3[d], base = id - c3[d] * s;
+            const int c = c3[d];
+            auto diff = [&](int p) {
+                const long q = base + (p == 0 ? 1 : p) * s;
+                return a.src[q] - a.src[q - s];
+            };
+            double am, bp;
+            if (c >= 2 && c <= L3[d] - 4) {
+                double v[6];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) v[k] = diff(c - 2 + k);
+                const double A0 = v[1] - v[0], A1 = v[2] - v[1], A2 = v[3] - v[2], A3 = v[4] - v[3], A4 = v[5] - v[4];
+                both_sides(v[2], v[3], A0, A1, A2, A3, A4, kSqrt13_3 * (A1 - A0), kSqrt13_3 * (A2 - A1),
+                           kSqrt13_3 * (A3 - A2), kSqrt13_3 * (A4 - A3), eps, am, bp);
+            } else {
+                int p[5];
+                double v[5];
+                stencil_left(c, L3[d], p);
+                for (int k = 0; k < 5; ++k) v[k] = diff(p[k]);
+                if (d == 2 && a.ref_bugs && c == nzg - 1) {
+                    // lsTools.cu:636: id_kp2 = id_jm1 at the top layer
+                    const long ib = c3[1] == 0 ? id : id - nxg;
+                    v[4] = a.src[ib] - a.src[ib - sxy];
+                }
+                am = weno5(v[0], v[1], v[2], v[3], v[4], eps);
+                stencil_right(c, L3[d], p);
+                for (int k = 0; k < 5; ++k) v[k] = diff(p[k]);
+                bp = weno5(v[0], v[1], v[2], v[3], v[4], eps);
+            }
+            // Godunov, as in k_reinit_stage
+            am *= C;
+            bp *= C;
+            const double m1 = larger(pos_part(am), neg_mag(bp)), m2 = larger(pos_part(bp), neg_mag(am));
+            r += tsg > 0 ? m1 * m1 : (tsg < 0 ? m2 * m2 : fma(0.5, m2 * m2, 0.5 * (m1 * m1)));
+        }
+        const double dm = a.dmins[id];
+        const double rs = (p0 * rsqrt_fast(fma(p0, p0, dm * dm))) * (sqrt_fast(r) - 1.0);
+        const double t = a.src[id] - a.dt * rs;
+        double o;
+        if (a.stage == 1) o = t;
+        else if (a.stage == 2) o = 0.75 * a.phi[id] + 0.25 * t;
+        else o = fma(2.0, t, a.phi[id]) * (1.0 / 3.0);
+        a.out[id] = o;
+    }
+}
+
 // ghost layers of a padded field from its own interior (mirror images)
 __global__ void k_mirror_inplace(double *f, int g, int nx, int ny, int nz) {
     const int nxg = nx + 2 * g, nyg = ny + 2 * g, nzg = nz + 2 * g;
@@ -260,34 +325,56 @@ int grid_r(long n) { return grid_cap(n, 8); }
 
 } // namespace
 
+// Whether the stages go by cells: where a launch's grid does not reach, and on
+// small grids whose one-plane blocks are a few more than one for each SM, or than
+// the three an SM holds, so that a second one or round runs for those few, while
+// the cells by themselves are less (one block of theirs an SM, or the second
+// round).  ms a call of 10 iterations, marching / by cells: 30 x 30 x 40 1.43 /
+// 1.12, 37 x 50 x 42 2.48 / 1.97, 49 x 50 x 30 2.24 / 1.86; 55 x 55 x 35 2.45 / 2.8.
+static bool by_cells(long cols, int gy, int nzg, long ng) {
+    const long sms = device_sms(), blocks = cols * nzg;
+    return gy > 65535 || (blocks > sms && ng <= 256 * sms) || (blocks > 3 * sms && blocks <= 4 * sms && ng < 600 * sms);
+}
+
 int reinit_impl(double *phi, const double *jbn, const double *dmins, double dX, double dY, double dZ,
                 int nxg, int nyg, int nzg, int g, double deltamin, int iters, int ref_bugs,
                 cudaStream_t st) {
     const long ng = (long)nxg * nyg * nzg;
+    const int gx = (nxg + kMX - 1) / kMX, gy = (nyg + kMY - 1) / kMY;
     double *scr;
-    int rc = device_scratch((size_t)9 * ng * sizeof(double), &scr);
+    bool cells = by_cells((long)gx * gy, gy, nzg, ng);
+    // a call whose nine fields do not fit goes by cells, in two
+    int rc = device_scratch((size_t)(cells ? 2 : 9) * ng * sizeof(double), &scr);
+    if (rc == EMIX_ERR_ALLOC && !cells) {
+        cells = true;
+        rc = device_scratch((size_t)2 * ng * sizeof(double), &scr);
+    }
     if (rc) return rc;
-    double *A = scr + 6 * ng, *B = scr + 7 * ng;
+    double *A = cells ? scr : scr + 6 * ng, *B = A + ng;   // the pairs first, 16-byte aligned
     const int nx = nxg - 2 * g, ny = nyg - 2 * g, nz = nzg - 2 * g;
     ReinitArgs a{};
     a.phi = phi; a.dmins = dmins;
-    a.ce = reinterpret_cast<const double2 *>(scr);
-    a.sgn = scr + 8 * ng;
     a.nxg = nxg; a.nyg = nyg; a.nzg = nzg;
     a.dt = 0.5 * deltamin; a.ref_bugs = ref_bugs;
-    const int gx = (nxg + kMX - 1) / kMX, gy = (nyg + kMY - 1) / kMY;
-    if (gy > 65535) return EMIX_ERR_ARG;
-    const int gz = march_chunks((long)gx * gy, nzg, 3);
-    const dim3 grid(gx, gy, gz);
-    k_reinit_scales<<<grid_r(ng), 256, 0, st>>>(jbn, reinterpret_cast<double2 *>(scr), 1.0 / dX, 1.0 / dY, 1.0 / dZ, ng);
+    dim3 grid(1);
+    if (!cells) {
+        a.ce = reinterpret_cast<const double2 *>(scr);
+        a.sgn = B + ng;
+        grid = dim3(gx, gy, march_chunks((long)gx * gy, nzg, 3));
+        k_reinit_scales<<<grid_r(ng), 256, 0, st>>>(jbn, reinterpret_cast<double2 *>(scr), 1.0 / dX, 1.0 / dY, 1.0 / dZ, ng);
+    }
+    auto stage = [&](int q, const double *src, double *out) {
+        a.src = src;
+        a.out = out;
+        a.stage = q;
+        if (cells) k_reinit_cells<<<grid_r(ng), 256, 0, st>>>(a, jbn, 1.0 / dX, 1.0 / dY, 1.0 / dZ);
+        else k_reinit_stage<<<grid, kNT, 0, st>>>(a);
+    };
     for (int it = 0; it < iters; ++it) {
         if (g > 0) k_mirror_inplace<<<grid_r(ng), 256, 0, st>>>(phi, g, nx, ny, nz);
-        a.src = phi; a.out = A; a.stage = 1;
-        k_reinit_stage<<<grid, kNT, 0, st>>>(a);
-        a.src = A; a.out = B; a.stage = 2;
-        k_reinit_stage<<<grid, kNT, 0, st>>>(a);
-        a.src = B; a.out = phi; a.stage = 3;
-        k_reinit_stage<<<grid, kNT, 0, st>>>(a);
+        stage(1, phi, A);
+        stage(2, A, B);
+        stage(3, B, phi);
     }
     EMIX_CUDA_TRY(cudaGetLastError());
     return EMIX_OK;

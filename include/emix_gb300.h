@@ -264,7 +264,8 @@ int emix_deriv_t_tma_dev(int scheme, int axis, int nf, double *out, const double
  * gcells ghost layers, mirrored at the start of every iteration; iters
  * iterations (10 in the reference) of three TVD-RK3 stages of deltamin/2; the
  * kernels use 1/deltaX.  ref_bugs keeps the z-top index of
- * PhiDevPlusParameterJB.  Uses the library's per-device scratch. */
+ * PhiDevPlusParameterJB.  Uses the library's per-device scratch: nine padded
+ * fields, or two where nine do not fit (and on some small grids). */
 int emix_reinit_dev(double *phi, const double *jbn, const double *dmins, double deltaX, double deltaY,
                     double deltaZ, int nxg, int nyg, int nzg, int gcells, double deltamin, int iters,
                     int ref_bugs, void *stream);
