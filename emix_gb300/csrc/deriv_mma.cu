@@ -10,7 +10,9 @@
 // 1024, the operator into digits of the same kind, and the sums of digit products
 // are integers in f32 (the error-free splitting of K. Ozaki et al., Numerical
 // Algorithms 59, 2012, applied to a banded operator).  Products of digit orders
-// i + j <= 5 are kept.
+// i + j <= 5 are kept; the sums of the first four orders are below 2^24 and exact,
+// those of the last two round in the worst case, by 2^-54 of the result
+// (deriv_table.cu).
 //
 // Errors, relative to the pencil's largest difference over h: 2^-57 from the
 // products dropped, up to 2^-55.8 from the operator's cut at 40 rows.  The sweeps

@@ -728,7 +728,7 @@ int build_mma(int scheme, int n, double h, double sign, MmaTable &t, std::vector
         int lead[kMmaWin];
         for (int &l : lead) l = kMmaDig;
         for (int o = 0; o < kMmaRows; ++o) {
-            long size[3] = {0, 0, 0};   // sums of |digit| over the row, per leading digit
+            long size[kMmaDig] = {};   // sums of |digit| over the row, per digit
             real sum = 0;
             for (int k = 0; k < cnt; ++k) {
                 const real v = std::ldexp(E[(size_t)ty * kMmaRows + o][k], t.se);
@@ -746,19 +746,21 @@ int build_mma(int scheme, int n, double h, double sign, MmaTable &t, std::vector
                 const int g = k / kMmaRows, kk = k % kMmaRows;
                 for (int i = 0; i < kMmaDig; ++i) {
                     if (d[i] && i < lead[g]) lead[g] = i;
-                    if (i < 3) size[i] += std::abs(d[i]);
+                    size[i] += std::abs(d[i]);
                     b[((size_t)ty * kMmaTypeBytes + g * kMmaGroupBytes + (kk / 8) * (kMmaStack * 16) +
                        (i * kMmaRows + o) * 16) / 2 + kk % 8] = half_bits(d[i]);
                 }
             }
-            // the f32 sums of the three leading digit orders are exact integers
-            // (the lower orders' worst case, all digits at their bound and of one
-            // sign, exceeds 2^24 by up to 2, costing 2^-48 of the result), and
-            // the combined sum fits 64 bits
+            // the f32 sums of the first four digit orders stay below 2^24, where every
+            // integer is exact; in the worst case (all of a pencil's digits at their
+            // bound and of one sign) those of the fifth reach 1.4 x 2^24 and of the
+            // sixth 2.1 x, where sums round to even units and to multiples of four: 28
+            // such roundings are 2^-54 of the largest result.  The combined sum fits 64
+            // bits.
             long s = 0;
-            for (int i = 0; i < 3; ++i) {
+            for (int i = 0; i < kMmaDig; ++i) {
                 s += size[i] * 512;
-                if (s >= 1L << 24) return EMIX_ERR_UNSUPPORTED;
+                if (s >= 1L << (i < 4 ? 24 : 21 + i)) return EMIX_ERR_UNSUPPORTED;
             }
             if (sum > 4000 * std::ldexp(real(1), 10 * (kMmaDig - 1))) return EMIX_ERR_UNSUPPORTED;
         }
