@@ -631,13 +631,21 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
                     prev = before;
                 }
                 int w = 0;
-#pragma unroll
-                for (int q = 0; q < kScan; ++q) {
-                    if (q >= rows) break;
+                auto take = [&](int q) {
                     const double d = sv[q] - prev;
                     prev = sv[q];
                     w = max(w, size_of(d));
                     low |= (unsigned)__double2loint(d);
+                };
+                if (rows == kScan) {
+#pragma unroll
+                    for (int q = 0; q < kScan; ++q) take(q);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kScan; ++q) {
+                        if (q >= rows) break;
+                        take(q);
+                    }
                 }
                 top = max(top, w);
                 if (window) least = min(least, w);
