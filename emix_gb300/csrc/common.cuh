@@ -53,12 +53,12 @@ inline int grid_cap(long n, int per_sm, int bs = 256) {
 EMIX_DEV void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>
-inline cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t shm, cudaStream_t st, A &&...args) {
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int block, size_t shm, cudaStream_t st, A &&...args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = shm;
     cfg.stream = st;
@@ -205,6 +205,13 @@ struct DerivTable {
     const double *u0s;     // ku weights of the scaled form: u0_k k_k (periodic)
     double sm1s;           // sm1 k_{n-1} (periodic)
     const struct MmaTable *mma;   // host: the same operator for the tensor cores (null: none)
+};
+
+// Which of a derivative's two forms runs, decided on the device from a sample of its
+// pencils (launch_quiet_sample, deriv_mma.cu): both are launched, one returns at once.
+struct QuietGate {
+    int sweeps;              // 1: the sweeps; 0: the tensor cores
+    int sum, done, pad;      // of the sample's blocks; 0 between its launches
 };
 
 // Parallel cyclic reduction (PCR) followed by Thomas, for one compact

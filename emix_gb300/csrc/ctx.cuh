@@ -17,6 +17,7 @@ struct emix_ctx {
     double *um0, *um, *u, *pres, *dvel, *vis, *amut, *vort, *flux, *R, *W, *jbn, *jx, *jy, *jz,
         *mask, *dxyz, *ratios, *phi, *phig0, *phigA, *phigB, *wenoCE, *xyz, *clock;
     unsigned char *impflag = nullptr;
+    emix::QuietGate *gates = nullptr;   // of the gradients along x, y, z, of the divergence likewise
     // blade-edge interpolation of the impeller (imp.interp)
     double *ip_geo = nullptr;
     unsigned char *ip_status = nullptr;

@@ -293,10 +293,18 @@ EMIX_DEV void deriv_yz_body(const DerivTable &T, const PencilFields &F, int nx, 
     deriv_pencil<EPI>(T, pick(F.in, f) + base, pick(F.w, f) + base, pick(F.out, f) + base, s);
 }
 
+// (of the sweeps, launched early then)
+EMIX_DEV bool gate_shut(const QuietGate *gate) {
+    if (!gate) return false;
+    wait_for_previous();
+    return !gate->sweeps;
+}
+
 // grid: (ceil(nx/blockDim.x), nother, nf); blockIdx.z = field
 template <int EPI>
 __global__ void __launch_bounds__(128)
-k_deriv_yz(DerivTable T, PencilFields F, int nx, int nother, long s, long os) {
+k_deriv_yz(DerivTable T, PencilFields F, int nx, int nother, long s, long os, const QuietGate *gate) {
+    if (gate_shut(gate)) return;
     deriv_yz_body<EPI>(T, F, nx, nother, s, os, blockIdx, threadIdx.x, blockDim.x);
 }
 
@@ -482,16 +490,18 @@ EMIX_DEV void deriv_x_body(const DerivTable &T, const PencilFields &F, long npen
 
 template <int EPI>
 __global__ void __launch_bounds__(128)
-k_deriv_x(DerivTable T, PencilFields F, long npencil) {
+k_deriv_x(DerivTable T, PencilFields F, long npencil, const QuietGate *gate) {
+    if (gate_shut(gate)) return;
     extern __shared__ double smem[];
     deriv_x_body<EPI>(T, F, npencil, blockIdx, threadIdx.x, blockDim.x >> 5, smem);
 }
 
 // Launch helper: derivative of nf fields along axis; w may equal out when
-// epi == EPI_STORE.  in must not alias w/out.
+// epi == EPI_STORE.  in must not alias w/out.  With a gate, it does nothing unless the
+// gate names its form.
 int launch_deriv(const DerivTable &T, int axis, int epi, int nf, const double *const *in,
                  double *const *w, double *const *out, int nx, int ny, int nz,
-                 cudaStream_t st);
+                 cudaStream_t st, const QuietGate *gate = nullptr);
 
 // Stored y and z derivatives in one launch (k_deriv_yz_pair): nfa fields
 // along axis 1 (in/out [0, nfa)), nfb along axis 2 (the next nfb); w = out.

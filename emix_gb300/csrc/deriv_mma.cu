@@ -463,7 +463,7 @@ EMIX_DEV void scan_x(const double *f, int p0, int np, int n, int uw, int step, i
 // otherwise along y or z (pencils contiguous along x)
 // CTA `cta` of the I.ncta that share the item
 template <bool XAX, int EPI, int KIND>
-EMIX_DEV void mma_body(const MmaItem &I, int cta) {
+EMIX_DEV void mma_body(const MmaItem &I, int cta, const QuietGate *gate) {
     constexpr bool PER = KIND == kCyclic || KIND == kRound;
     constexpr int kScanParts = scan_parts(XAX);
     const MmaTable &M = I.M;
@@ -528,7 +528,7 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     const int nblk = M.nblk;
     const int g0 = PER ? -2 : 0;                                   // first and last group of a tile
     const int g1 = PER ? nblk + 2 : (n + 6) / kMmaRows;
-    const int jobs = whole + (ntile * nf - whole) * segs;
+    int jobs = whole + (ntile * nf - whole) * segs;
     constexpr bool round = KIND == kRound;
     constexpr int kOutTiles = out_tiles(KIND);
     bool ok = true;                                                // false: a wait ran out; nothing is stored any more
@@ -698,7 +698,8 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     };
     constexpr int kPencilWarps = 2 * kRoleWarps + kScanWarps;   // all but the tensor core's
     wait_for_previous();   // what is read so far is constant
-    if (warp != 2 * kRoleWarps) {
+    if (gate && gate->sweeps) jobs = 0;   // nothing to do, past the setup
+    if (warp != 2 * kRoleWarps && jobs > 0) {
         // the first tile's, by all of them
         scan_tile(cta, 0, warp < 2 * kRoleWarps ? warp : warp - 1, kPencilWarps);
     }
@@ -1070,9 +1071,73 @@ EMIX_DEV void mma_body(const MmaItem &I, int cta) {
     }
 }
 
+// 32 neighbouring pencils a block, each group's `every`-th: which of them are quiet
+// somewhere (windows as of the scan, 16 rows or along x 32)
+template <bool XAX>
+__global__ void __launch_bounds__(256) k_quiet_sample(PencilFields F, int nf, int n, int np, int nx, long s, long os,
+                                                      int limit, QuietGate *gate) {
+    __shared__ int s_top[8][32], s_least[8][32];
+    wait_for_previous();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = (np + 31) / 32, id = (int)((long)blockIdx.x * per * nf / gridDim.x);
+    const int f = id / per, p0 = (id - f * per) * 32;
+    int top = 0, least = 0x7fffffff;
+    if constexpr (!XAX) {
+        const int p = min(p0 + lane, np - 1);
+        const double *in = pick(F.in, f) + p % nx + (long)(p / nx) * os;
+        for (int r = 16 * warp; r < n; r += 128) {
+            double prev = in[(long)max(r - 1, 0) * s], v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = in[(long)min(r + q, n - 1) * s];
+            int w = 0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                w = max(w, size_of(v[q] - prev));
+                prev = v[q];
+            }
+            top = max(top, w);
+            if (r + 16 <= n) least = min(least, w);
+        }
+        s_top[warp][lane] = top;
+        s_least[warp][lane] = least;
+    } else {
+        for (int q = warp; q < 32; q += 8) {
+            const double *in = pick(F.in, f) + (long)min(p0 + q, np - 1) * n;
+            int t = 0, l = 0x7fffffff;
+            for (int r0 = 0; r0 < n; r0 += 32) {
+                const int r = min(r0 + lane, n - 1);
+                const int w = __reduce_max_sync(0xffffffffu, size_of(in[r] - in[max(r - 1, 0)]));
+                t = max(t, w);
+                if (r0 + 32 <= n) l = min(l, w);
+            }
+            if (lane < 8) {
+                s_top[lane][q] = t;
+                s_least[lane][q] = l;
+            }
+        }
+    }
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        top = max(top, s_top[q][lane]);
+        least = min(least, s_least[q][lane]);
+    }
+    const unsigned quiet = __ballot_sync(0xffffffffu, p0 + lane < np && top - least > kMmaSpan << 20);
+    if (lane == 0) {
+        atomicAdd(&gate->sum, __popc(quiet));
+        __threadfence();
+        if (atomicAdd(&gate->done, 1) == (int)gridDim.x - 1) {   // the last block
+            __threadfence();
+            gate->sweeps = atomicExch(&gate->sum, 0) > limit;
+            gate->done = 0;
+        }
+    }
+}
+
 template <bool XAX, int EPI, int KIND>
 __global__ void __launch_bounds__(kMmaThreads, 1) k_deriv_mma(const __grid_constant__ MmaItem I) {
-    mma_body<XAX, EPI, KIND>(I, blockIdx.x);
+    mma_body<XAX, EPI, KIND>(I, blockIdx.x, I.gate);
 }
 
 // many grids' derivatives: the SMs are divided between the items (mma_split)
@@ -1088,7 +1153,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_batch_deriv_mma(const MmaIte
     for (int q = threadIdx.x; q < (int)(sizeof(MmaItem) / sizeof(int)); q += kMmaThreads)
         reinterpret_cast<int *>(&s_item)[q] = reinterpret_cast<const int *>(items + g)[q];
     __syncthreads();
-    mma_body<XAX, EPI, KIND>(s_item, (int)blockIdx.x - s_item.cta0);
+    mma_body<XAX, EPI, KIND>(s_item, (int)blockIdx.x - s_item.cta0, nullptr);
 }
 
 // tensor memory is taken whole: at least 116 KB of shared memory keeps a
@@ -1200,10 +1265,32 @@ static PencilFields fields_of(int nf, const double *const *in, double *const *w,
 }
 
 int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
-                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st) {
+                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st,
+                     const QuietGate *gate) {
     MmaItem I = mma_item(T, M, axis, fields_of(nf, in, w, out), nf, nx, ny, nz);
+    I.gate = gate;
     divide(I, device_sms());
     return launch_variant(axis == 0, epi, kind_of(T.n, M.periodic != 0), I, st);
+}
+
+int launch_quiet_sample(int axis, int nf, const double *const *in, int nx, int ny, int nz, QuietGate *gate,
+                        cudaStream_t st) {
+    PencilFields F{};
+    for (int f = 0; f < nf; ++f) F.in[f] = in[f];
+    const int n = axis == 0 ? nx : (axis == 1 ? ny : nz), np = axis == 0 ? ny * nz : nx * (axis == 1 ? nz : ny);
+    const long s = axis == 1 ? (long)nx : (long)nx * ny, os = axis == 1 ? (long)nx * ny : (long)nx;
+    const int groups = (np + 31) / 32 * nf, sms = device_sms(), blocks = std::min(groups, 2 * sms);
+    // A launch gains 5 to 8 ps a cell and field over the sweeps; the quiet pencils of an
+    // SM, once more than its warps take one by one, cost it a thread's walk, 0.6 to 1.2
+    // us a row.  1200 pencils an SM is where a launch gains the walk: with more, a fifth
+    // of them may be quiet (256^3, ms, 5 fields: x 0.82 at 10%, 1.17 at 30%, sweeps 1.00;
+    // y 0.89, 1.03, 0.99), with fewer, as many as the warps take (128^3: x 0.10 at 1%,
+    // 0.17 at 10%, sweeps 0.15; y 0.09, 0.17, 0.17).
+    const long all = (long)np * nf, most = all >= 1200L * sms ? all / 5 : (long)kSweepWarps * std::max(1, n / 96) * sms;
+    const int limit = (int)(most * 32 * blocks / all);
+    auto kernel = axis == 0 ? k_quiet_sample<true> : k_quiet_sample<false>;
+    EMIX_CUDA_TRY(launch_early(kernel, blocks, 256, 0, st, F, nf, n, np, nx, s, os, limit, gate));
+    return EMIX_OK;
 }
 
 int deriv_mma_timeouts(int *count) {

@@ -64,7 +64,22 @@ inline bool deriv_on_mma(const DerivTable &T) { return T.mma != nullptr; }
 
 // launch_deriv on the tensor cores
 int launch_deriv_mma(const DerivTable &T, const MmaTable &M, int axis, int epi, int nf, const double *const *in,
-                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st);
+                     double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st,
+                     const QuietGate *gate = nullptr);
+
+// Sets `gate` from a sample of the pencils: to the sweeps where more of them are
+// quiet somewhere than the tensor cores' form gains from (those take a sweep there
+// too, after a scan, and less well spread over the SM).
+int launch_quiet_sample(int axis, int nf, const double *const *in, int nx, int ny, int nz, QuietGate *gate,
+                        cudaStream_t st);
+// Cells of a step's grid from which its derivatives are gated.  A step then has 24
+// launches more, 0.12 ms (ms, ungated / gated: tanks in motion 128^3 4.19 / 4.31, 160^3
+// 7.63 / 7.75, 256^3 28.10 / 28.25), which the states with many quiet pencils repay:
+// a tank from rest 128^3 5.1-6.2 / 4.9-5.2, 256^3 36-43.6 / 33-33.8; bench.py's after 125
+// steps 37.8 / 33.8 (the sweeps everywhere: 5.05, 34.5, 34.7).  Smaller grids would pay more
+// than the states that last gain: 96^3 in motion 2.05 / 2.15, developed 2.32 / 2.32, from
+// rest 2.6-3.2 / 2.4-2.7 (sweeps 2.56).
+constexpr long kGateCells = 1L << 21;
 
 // One derivative of nf fields of a grid, and the CTAs that walk its tiles.
 struct MmaItem {
@@ -75,6 +90,7 @@ struct MmaItem {
     int whole, segs;          // whole tiles, and segments each of the others is cut into
     int cta0, ncta;           // CTAs [cta0, cta0 + ncta) of the launch
     long s, os;               // strides along a pencil, and between lines of pencils
+    const QuietGate *gate;    // null: none
 };
 MmaItem mma_item(const DerivTable &T, const MmaTable &M, int axis, const PencilFields &F, int nf, int nx, int ny,
                  int nz);

@@ -51,12 +51,12 @@ int yz_block(int nx) {
 }
 
 int launch_deriv(const DerivTable &T, int axis, int epi, int nf, const double *const *in,
-                 double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st) {
+                 double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st, const QuietGate *gate) {
     if (nf < 1 || nf > kMaxFields) return EMIX_ERR_ARG;
     const int n = axis == 0 ? nx : (axis == 1 ? ny : nz);
     if (T.n != n) return EMIX_ERR_ARG;
     if (deriv_on_mma(T))
-        return launch_deriv_mma(T, *T.mma, axis, epi, nf, in, w, out, nx, ny, nz, st);
+        return launch_deriv_mma(T, *T.mma, axis, epi, nf, in, w, out, nx, ny, nz, st, gate);
     PencilFields F{};
     for (int f = 0; f < nf; ++f) {
         F.in[f] = in[f];
@@ -69,10 +69,9 @@ int launch_deriv(const DerivTable &T, int axis, int epi, int nf, const double *c
         const long blocks = (np + 32 * warps - 1) / (32 * warps);
         const size_t shm = (size_t)warps * kXTile * sizeof(double);
         dim3 grid((unsigned)blocks, 1, nf);
-        if (epi == EPI_STORE)
-            k_deriv_x<EPI_STORE><<<grid, 32 * warps, shm, st>>>(T, F, np);
-        else
-            k_deriv_x<EPI_ACCUM><<<grid, 32 * warps, shm, st>>>(T, F, np);
+        auto kernel = epi == EPI_STORE ? k_deriv_x<EPI_STORE> : k_deriv_x<EPI_ACCUM>;
+        if (gate) EMIX_CUDA_TRY(launch_early(kernel, grid, 32 * warps, shm, st, T, F, np, gate));
+        else kernel<<<grid, 32 * warps, shm, st>>>(T, F, np, gate);
     } else {
         const int bs = yz_block(nx);
         const int nother = axis == 1 ? nz : ny;
@@ -80,10 +79,9 @@ int launch_deriv(const DerivTable &T, int axis, int epi, int nf, const double *c
         const long os = axis == 1 ? (long)nx * ny : (long)nx;
         if (nother > 65535) return EMIX_ERR_ARG;
         dim3 grid((nx + bs - 1) / bs, nother, nf);
-        if (epi == EPI_STORE)
-            k_deriv_yz<EPI_STORE><<<grid, bs, 0, st>>>(T, F, nx, nother, s, os);
-        else
-            k_deriv_yz<EPI_ACCUM><<<grid, bs, 0, st>>>(T, F, nx, nother, s, os);
+        auto kernel = epi == EPI_STORE ? k_deriv_yz<EPI_STORE> : k_deriv_yz<EPI_ACCUM>;
+        if (gate) EMIX_CUDA_TRY(launch_early(kernel, grid, bs, 0, st, T, F, nx, nother, s, os, gate));
+        else kernel<<<grid, bs, 0, st>>>(T, F, nx, nother, s, os, gate);
     }
     EMIX_CUDA_TRY(cudaGetLastError());
     return EMIX_OK;

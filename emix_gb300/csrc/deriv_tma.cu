@@ -410,7 +410,8 @@ EMIX_DEV void tma_pencils_t(const CUtensorMap *mi, const CUtensorMap *mw, const 
 template <int B, int EPI, bool CYC>
 __global__ void __launch_bounds__(B)
 k_deriv_yz_tma(const __grid_constant__ PencilMaps M, const DerivTable Ta, const DerivTable Tb,
-               const PencilFields F, int nfa, int nx, int ny, int nz) {
+               const PencilFields F, int nfa, int nx, int ny, int nz, const QuietGate *gate) {
+    if (gate_shut(gate)) return;
     __shared__ __align__(128) double buf[kPtS * 2 * kPtR * B];
     __shared__ __align__(8) unsigned long long bar[kPtS];
     __shared__ int s_ok[2];
@@ -504,7 +505,7 @@ bool pencil_tma_maps(PencilMaps *M, const int *axis, int nf, const double *const
 
 int launch_deriv_yz_tma(const DerivTable &Ta, const DerivTable &Tb, const PencilMaps &M, int epi, int nfa, int nf,
                         const double *const *in, double *const *w, double *const *out, int nx, int ny, int nz,
-                        cudaStream_t st) {
+                        cudaStream_t st, const QuietGate *gate) {
     if (nf < 1 || nf > kMaxFields || nfa < 0 || nfa > nf || (epi != EPI_STORE && epi != EPI_ACCUM)) return EMIX_ERR_ARG;
     // one launch is all closed or all cyclic tables
     const bool cyc = (nfa > 0 ? Ta : Tb).periodic != 0;
@@ -528,10 +529,13 @@ int launch_deriv_yz_tma(const DerivTable &Ta, const DerivTable &Tb, const Pencil
     const dim3 grid((nx + B - 1) / B, nother, nf);
 #define EMIX_TMA_LAUNCH(BW, CY)                                                                     \
     if (B == BW && cyc == CY) {                                                                     \
-        if (epi == EPI_ACCUM)                                                                       \
-            k_deriv_yz_tma<BW, EPI_ACCUM, CY><<<grid, BW, 0, st>>>(M, Ta, Tb, F, nfa, nx, ny, nz);  \
-        else                                                                                        \
-            k_deriv_yz_tma<BW, EPI_STORE, CY><<<grid, BW, 0, st>>>(M, Ta, Tb, F, nfa, nx, ny, nz);  \
+        auto kernel = epi == EPI_ACCUM ? k_deriv_yz_tma<BW, EPI_ACCUM, CY>                          \
+                                       : k_deriv_yz_tma<BW, EPI_STORE, CY>;                         \
+        if (gate) {                                                                                 \
+            EMIX_CUDA_TRY(launch_early(kernel, grid, BW, 0, st, M, Ta, Tb, F, nfa, nx, ny, nz, gate)); \
+            return EMIX_OK;                                                                         \
+        }                                                                                           \
+        kernel<<<grid, BW, 0, st>>>(M, Ta, Tb, F, nfa, nx, ny, nz, gate);                           \
         EMIX_CUDA_TRY(cudaGetLastError());                                                          \
         return EMIX_OK;                                                                             \
     }

@@ -42,10 +42,10 @@ bool pencil_tma_maps(PencilMaps *M, const int *axis, int nf, const double *const
 // D in along each field's axis, rows staged by TMA through the maps M:
 // out += D in (EPI_ACCUM) or out = D in (EPI_STORE, w = out); fields [0, nfa)
 // with table Ta, the rest with Tb (fields as in launch_deriv), the tables
-// all closed or all cyclic.
+// all closed or all cyclic.  With a gate as launch_deriv.
 int launch_deriv_yz_tma(const DerivTable &Ta, const DerivTable &Tb, const PencilMaps &M, int epi, int nfa, int nf,
                         const double *const *in, double *const *w, double *const *out, int nx, int ny, int nz,
-                        cudaStream_t st);
+                        cudaStream_t st, const QuietGate *gate = nullptr);
 
 // D^T in along each field's axis (a closed table T), rows staged by TMA
 // through the maps M: out = D^T in (acc = 0) or out += D^T in (acc = 1), with

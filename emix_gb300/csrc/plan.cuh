@@ -56,6 +56,8 @@ struct Launch {
     };
     const CUtensorMap *tmap;   // LK_WENO: plane tiles by TMA (null: register-staged loads)
     const PencilMaps *pmaps;   // LK_DERIV_YZ accumulating: rows by TMA (null: loads)
+    QuietGate *gate;           // LK_DERIV_X, _YZ on the tensor cores of large grids: they or the sweeps
+    bool sample;               // (this record sets it)
     const PencilMaps *pair_pmaps;   // the gradients' y record: the fused y + z launch by TMA
 };
 

@@ -25,9 +25,6 @@
 #include <vector>
 
 namespace emix {
-int launch_deriv(const DerivTable &T, int axis, int epi, int nf, const double *const *in,
-                 double *const *w, double *const *out, int nx, int ny, int nz, cudaStream_t st);
-
 __global__ void k_metric_products(const double *__restrict__ jbn, double *__restrict__ jx,
                                   double *__restrict__ jy, double *__restrict__ jz, long n) {
     EMIX_FOR_CELLS(q, n) {
@@ -37,6 +34,22 @@ __global__ void k_metric_products(const double *__restrict__ jbn, double *__rest
         jz[q] = j10 * jbn[8 * n + q];
     }
 }
+// launches of a record
+static int launches_of(const Launch &L) { return L.gate ? 2 + L.sample : 1; }
+
+// a derivative in both forms, of which the gate lets one run
+static int launch_gated(const Launch &L, cudaStream_t st) {
+    const DerivArgs &a = L.deriv;
+    int rc = L.sample ? launch_quiet_sample(a.axis, a.nf, a.F.in, a.nx, a.ny, a.nz, L.gate, st) : EMIX_OK;
+    if (!rc) rc = launch_deriv(a.T, a.axis, a.epi, a.nf, a.F.in, a.F.w, a.F.out, a.nx, a.ny, a.nz, st, L.gate);
+    if (rc) return rc;
+    DerivTable T = a.T;
+    T.mma = nullptr;
+    if (L.pmaps)
+        return launch_deriv_yz_tma(T, T, *L.pmaps, a.epi, a.nf, a.nf, a.F.in, a.F.w, a.F.out, a.nx, a.ny, a.nz, st, L.gate);
+    return launch_deriv(T, a.axis, a.epi, a.nf, a.F.in, a.F.w, a.F.out, a.nx, a.ny, a.nz, st, L.gate);
+}
+
 int launch_single(const Launch &L, cudaStream_t st) {
     switch (L.kind) {
     case LK_PRIM:
@@ -50,6 +63,7 @@ int launch_single(const Launch &L, cudaStream_t st) {
         return launch_weno_stage(L.weno, st, L.tmap);
     case LK_DERIV_X:
     case LK_DERIV_YZ:
+        if (L.gate) return launch_gated(L, st);
         if (L.pmaps && !deriv_on_mma(L.deriv.T))
             return launch_deriv_yz_tma(L.deriv.T, L.deriv.T, *L.pmaps, L.deriv.epi, L.deriv.nf, L.deriv.nf,
                                        L.deriv.F.in, L.deriv.F.w, L.deriv.F.out, L.deriv.nx, L.deriv.ny,
@@ -183,6 +197,14 @@ void build_plan(emix_ctx *c) {
     }
     for (int s = 1; s <= 3; ++s) {
         const double *umcur = s == 1 ? c->um0 : c->um;
+        // a derivative on the tensor cores, on large grids: they or the sweeps (sampled
+        // in the first substep, for all three)
+        auto gated = [&](int q) {
+            Launch &L = P.back();
+            if (n < kGateCells || !deriv_on_mma(L.deriv.T)) return;
+            L.gate = c->gates + q;
+            L.sample = s == 1;
+        };
         if (p.level_set) {
             Launch L = make(LK_WENO, CLS_WENO);
             WenoArgs &a = L.weno;
@@ -219,6 +241,7 @@ void build_plan(emix_ctx *c) {
             double *out[3] = {c->dvel + 3 * ax * n, c->dvel + (3 * ax + 1) * n, c->dvel + (3 * ax + 2) * n};
             P.push_back(deriv_launch(c->T[ax], ax, EPI_STORE, 3, in, out, out, nx, ny, nz, CLS_GRADX + ax));
             if (ax == 1) P.back().deriv.pair = 1;
+            gated(ax);
         }
         {
             // the y and z records as one launch with its rows by TMA, where
@@ -278,6 +301,7 @@ void build_plan(emix_ctx *c) {
                     pencil_tma_maps(pm, axes, 5, in, wb, out, nx, ny, nz))
                     P.back().pmaps = pm;
             }
+            gated(3 + ax);
         }
         // RK update and conversions; with walls the boundary conditions go
         // between the RK combination and the conversions (rungek_ico.f90:98-104):
@@ -334,6 +358,10 @@ static bool pair_apart(const std::vector<Launch> &P, size_t k) {
     return deriv_on_mma(P[k].deriv.T) || deriv_on_mma(P[k + 1].deriv.T);
 }
 
+static int launches_of_pair(const std::vector<Launch> &P, size_t k, int fuse) {
+    return fuse == 1 && pair_apart(P, k) ? launches_of(P[k]) + launches_of(P[k + 1]) : 1;
+}
+
 // Records k and k+1 of a plan that run as one launch: the gradients' y and z
 // records (1), Smagorinsky and the fluxes that read its viscosity (2); 0
 // otherwise.  The records stay separate in the plan: the fused kernels run
@@ -361,9 +389,8 @@ int launch_fused_pair(const std::vector<Launch> &P, size_t k, cudaStream_t st) {
         for (int f = 0; f < a.nf; ++f) { in[f] = a.F.in[f]; out[f] = a.F.out[f]; }
         for (int f = 0; f < b.nf; ++f) { in[a.nf + f] = b.F.in[f]; out[a.nf + f] = b.F.out[f]; }
         if (pair_apart(P, k)) {
-            int rc = launch_deriv(a.T, a.axis, EPI_STORE, a.nf, in, out, out, a.nx, a.ny, a.nz, st);
-            if (!rc) rc = launch_deriv(b.T, b.axis, EPI_STORE, b.nf, in + a.nf, out + a.nf, out + a.nf, a.nx, a.ny, a.nz, st);
-            return rc;
+            const int rc = launch_single(L, st);
+            return rc ? rc : launch_single(P[k + 1], st);
         }
         if (L.pair_pmaps)
             return launch_deriv_yz_tma(a.T, b.T, *L.pair_pmaps, EPI_STORE, a.nf, a.nf + b.nf, in, out, out, a.nx,
@@ -414,7 +441,7 @@ int issue_step(emix_ctx *c) {
             ProfScope ps(c, fuse == 1 ? CLS_GRADYZ : CLS_SGSFLUX);
             int rc = launch_fused(c, k, c->stream);
             if (rc) return rc;
-            launches += fuse == 1 && pair_apart(c->plan, k) ? 2 : 1;
+            launches += launches_of_pair(c->plan, k, fuse);
             ++k;
             continue;
         }
@@ -436,7 +463,7 @@ int issue_step(emix_ctx *c) {
         ProfScope ps(c, L.cls);
         int rc = launch_single(L, c->stream);
         if (rc) return rc;
-        ++launches;
+        launches += launches_of(L);
     }
     if (fork && !joined) EMIX_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->join_ev[s - 1], 0));
     if (!gjoined) EMIX_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->gjoin_ev[gs - 1], 0));
@@ -712,7 +739,7 @@ int step_host_one(emix_ctx *c, const double *um_in, const double *phi_in, double
         const int fuse = fused_with_next(c, (size_t)k);
         int rc = fuse ? launch_fused(c, (size_t)k, st) : launch_single(L, st);
         if (rc) return rc;
-        launches += fuse == 1 && pair_apart(c->plan, (size_t)k) ? 2 : 1;
+        launches += fuse ? launches_of_pair(c->plan, (size_t)k, fuse) : launches_of(L);
         k += fuse ? 1 : 0;
     }
     if (!joined) EMIX_CUDA_TRY(cudaStreamWaitEvent(st, c->join_ev[fs - 1], 0));
@@ -771,7 +798,8 @@ int emix_ctx_create(const emix_params *p, emix_ctx **out) {
     const long nb2 = imp && p->imp.interp ? (long)p->imp.nblades * p->nx * p->ny : 0;
     const size_t ip_words = nb2 ? 11 * nb2 + 2 * ((nb2 + 7) / 8) + nb2 + (nb2 + 1) / 2 + kImpMaxBlades : 0;
     const size_t bytes = ((size_t)(nfield + (imp ? 3 : 0)) * n + 3 * (size_t)ng +
-                          (imp ? kImpClockLen + (n + 7) / 8 : 0) + ip_words + 1) * sizeof(double);
+                          (imp ? kImpClockLen + (n + 7) / 8 : 0) + ip_words + 1) * sizeof(double) +
+                         6 * sizeof(QuietGate);
     if (cudaMalloc(&c->arena, bytes) != cudaSuccess) {
         cudaGetLastError();
         set_last_message("cudaMalloc of the context arena failed");
@@ -785,6 +813,7 @@ int emix_ctx_create(const emix_params *p, emix_ctx **out) {
     c->dvel = take(9 * n); c->vis = take(n); c->flux = take(15 * n); c->R = take(5 * n);
     c->W = take(5 * n); c->jbn = take(11 * n); c->jx = take(n); c->jy = take(n); c->jz = take(n);
     c->mask = take(n); c->dxyz = take(n);
+    c->gates = reinterpret_cast<QuietGate *>(take(6 * sizeof(QuietGate) / sizeof(double)));
     c->phi = p->level_set ? take(n) : nullptr;
     if ((q - c->arena) & 1) ++q;   // 16-byte pairs
     c->wenoCE = p->level_set ? take(6 * n) : nullptr;
@@ -1151,13 +1180,13 @@ int emix_step_host(emix_ctx *c, double *um, double *phi, int nsteps) {
 
 int emix_ctx_launches_per_step(emix_ctx *c) {
     if (!c) return -1;
-    // every record is one launch, except the pairs that run as one
+    // every record is one launch, except the pairs that run as one and the gated ones
     int k = 0;
     const size_t np = c->plan.size();
     for (size_t q = 0; q < np; ++q) {
         const int fuse = fused_with_next(c, q);
-        if (fuse && !(fuse == 1 && pair_apart(c->plan, q))) ++q;
-        ++k;
+        k += fuse ? launches_of_pair(c->plan, q, fuse) : launches_of(c->plan[q]);
+        if (fuse) ++q;
     }
     return k;
 }

@@ -9,7 +9,8 @@
  * more are sums of integer digit products on the tensor cores, within 2^-55 of a
  * pencil's largest difference over the spacing (in the norm of a smooth pencil no
  * more than an FP64 solve's error).  Pencils in which some 32 rows differ by less
- * than 2^-10 of that, and infinities and NaN, are solved in FP64.
+ * than 2^-10 of that, and infinities and NaN, are solved in FP64; so is, in a context's
+ * step on 2^21 cells and more, every pencil of fields in which many are (by a sample).
  *
  * Two families of entry points:
  *   - the reference's own symbols (cudaDeriv, cuDivergence) with byte-identical
