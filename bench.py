@@ -99,10 +99,11 @@ IMPELLER = True
 # FP64 operations (dfma + dadd + dmul thread instructions) per cell a launch
 # covers, measured with ncu on the 192^3 tank (profiles/step_tensor_cores_
 # stirred_tank_192.txt; the unfused sgs and flux from their source).  The
-# derivatives run on the tensor cores: theirs is the accumulating add.
+# derivatives run on the tensor cores: theirs are the scan's differences, the
+# accumulating adds and the sweeps of the few pencils left to them.
 FP64_OPS_PER_CELL = {
-    "weno_stage": 113.0, "grad_x": 0.0, "grad_y": 0.0, "grad_z": 0.0, "grad_yz": 0.0,
-    "div_x": 0.0, "div_y": 5.0, "div_z": 5.0, "flux": 40.0, "sgs": 28.0, "sgs_flux": 55.0,
+    "weno_stage": 113.0, "grad_x": 4.0, "grad_y": 3.1, "grad_z": 3.0, "grad_yz": 6.1,
+    "div_x": 7.0, "div_y": 10.4, "div_z": 10.7, "flux": 40.0, "sgs": 28.0, "sgs_flux": 55.0,
     # the RK update: 22.3 in substep 1, 27.5 in substeps 2 and 3 (their um term)
     "rk_post": 25.8,
 }

@@ -53,12 +53,14 @@ struct MmaTable {
 int get_mma_table(int scheme, int n, double h, double sign, const MmaTable **out);
 
 // Whether a derivative goes to the tensor cores: by the length of its
-// pencils.  Measured against the sweeps (us a launch, 3 or 5 fields, closed /
-// cyclic): n = 32: x 17 / 21 -> 16 / 18 at 32^3 but 134 -> 200 at 32 x 128 x
-// 512, y and z 16 / 19 -> 16 / 19; n = 40: 26 / 33 -> 21 / 21, 22 / 25 -> 20 / 23;
-// n = 64: 36 / 47 -> 29 / 34, 33 / 38 -> 26 / 36; n = 256: 1001 / 1215 -> 694 /
-// 704, 991 / 1070 -> 577 / 710.  Shorter pencils have more blocks at an end and
-// groups to convert per output than the sweeps have to lose.
+// pencils.  Measured against the sweeps (us for 5 fields, closed / cyclic, x and y):
+// n = 40 on 48 x 48 pencils x 25 / 31 -> 17 / 19, y 19 / 23 -> 17 / 17, on 256 x 256
+// x 177 / 220 -> 145 / 202, y 152 / 192 -> 125 / 204 (the one loss); n = 64 x 33 / 43 ->
+// 18 / 18, y 27 / 33 -> 16 / 16, and 261 / 333 -> 170 / 187, 240 / 299 -> 155 / 159;
+// n = 256 x 1001 / 1212 -> 592 / 631, y 991 / 1071 -> 513 / 576.  n = 32, when the line
+// was drawn: x 17 / 21 -> 16 / 18 at 32^3 but 134 -> 200 at 32 x 128 x 512 (3 fields), y
+// and z 16 / 19 -> 16 / 19.  Shorter pencils have more blocks at an end and groups to
+// convert per output than the sweeps have to lose.
 constexpr int kMmaMinN = 40;
 inline bool deriv_on_mma(const DerivTable &T) { return T.mma != nullptr; }
 

@@ -121,7 +121,7 @@ EMIX_DEV void weno_z_general(const double *phi, long id, int Z, int nzg, bool le
 // (2.569); reinitialisation 70 x 81 x 32 1 (3.52, 2 planes 4.56), 106^3 3, 140 x 128
 // x 116 5.  Blocks of one plane that are a few more than are resident run a second
 // time for those few: two planes where that makes two blocks an SM
-// (reinitialisation 37 x 50 x 42: 2.78 -> 2.48).
+// (reinitialisation 37 x 50 x 42, before it went by cells: 2.78 -> 2.48).
 inline int march_chunks(long cols, int nz, int per_sm) {
     const long sms = device_sms();
     const double planes = (double)cols * nz / sms;
