@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 SIZES = [(128, 128, 128), (161, 96, 137), (2048, 40, 26)]
 
 
-def _work(dims, periodic, kind):
+def _state(dims, periodic, kind):
     """loud: waves and noise.  quiet: a bump of 1 over ripples of 1e-6 in every pencil
     of u, v and w.  half: the same and noise in every other pencil along x, so that
     pencils along y and z have it in every other row."""
@@ -48,7 +48,7 @@ def _gave_up(emix, ctx):
 @pytest.mark.parametrize("kind", ["loud", "quiet", "half"])
 @pytest.mark.parametrize("dims", SIZES)
 def test_values_and_forms(emix, dims, periodic, kind):
-    w = _work(dims, periodic, kind)
+    w = _state(dims, periodic, kind)
     b = emix.Batch([w], level_set=False)
     b.upload()
     b.step(2)
@@ -74,7 +74,7 @@ def test_the_sample_decides(emix):
     half's pencils)."""
     count = {}
     for kind in ("loud", "half"):
-        c = emix.Context(_work((128, 128, 128), False, kind), level_set=False)
+        c = emix.Context(_state((128, 128, 128), False, kind), level_set=False)
         count[kind] = _gave_up(emix, c)
         c.close()
     assert count["loud"] > 0 and count["half"] <= count["loud"] * 15 // 18
